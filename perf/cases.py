@@ -276,3 +276,108 @@ def tolerance(case):
     if case["kind"] == "indexer":
         return {"rel": 1e-6, "max": 1e-5}
     return {"rel": 7e-3, "max": 2e-2}
+
+
+def _scales(sf, col0, cols, k, gran):
+    """The float64 factor of every row of [col0, col0 + cols) and group of `gran` columns: byte j of word row r is group 4 r + j."""
+    words = sf[:, col0:col0 + cols].to(torch.int64) & 0xffffffff
+    e = torch.stack([(words >> (8 * j)) & 0xff for j in range(4)], dim=1).reshape(-1, cols)[:k // gran]
+    return torch.exp2(e.to(torch.float64) - 127.0).t()
+
+
+def _decode(dtype, codes, sf, col0, rows, k, gran):
+    """Rows [col0, col0 + rows) of a quantised operand as float64 values."""
+    raw = codes.view(torch.uint8).reshape(-1, k // 2 if dtype == Dtype.Fp4 else k)[col0:col0 + rows]
+    if dtype == Dtype.Fp4:
+        table = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, -0.0, -.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64, device=raw.device)
+        v = torch.stack([table[(raw & 15).long()], table[(raw >> 4).long()]], dim=-1).reshape(rows, k)
+    else:
+        v = raw.view(torch.float8_e4m3fn).to(torch.float64)
+    return (v.view(rows, k // gran, gran) * _scales(sf, col0, rows, k, gran)[:, :, None]).view(rows, k)
+
+
+def _rounded(x, dtype, gran):
+    """x after quantisation: every group of `gran` columns scaled by the smallest power of two that brings its largest
+    magnitude to the largest code or below, then rounded to the nearest code (ties to even)."""
+    m, k = x.shape
+    g = x.to(torch.float64).view(m, k // gran, gran)
+    top = 6.0 if dtype == Dtype.Fp4 else 448.0
+    s = torch.exp2(torch.ceil(torch.log2(g.abs().amax(dim=2, keepdim=True).clamp_min(1e-30) / top)))
+    v = g / s
+    if dtype == Dtype.Fp4:
+        step = torch.where(v.abs() < 2, 0.5, torch.where(v.abs() < 4, 1.0, 2.0)).to(torch.float64)
+        q = torch.round(v / step) * step
+    else:
+        q = v.to(torch.float32).to(torch.float8_e4m3fn).to(torch.float64)
+    return (q * s).view(m, k)
+
+
+def _relu_logits(q, kv, hw):
+    """sum_h hw[i, h] relu(<q[i, h], kv[j]>) for [i, h, d], [j, d] and [i, h]."""
+    s = torch.einsum("ihd,jd->ihj", q, kv).clamp_min_(0)
+    return torch.einsum("ihj,ih->ij", s, hw)
+
+
+def exact(case, seed):
+    """What `run` returns, in float64 from the same inputs.  The codes and scale words of the linear layers are whole
+    numbers that have no more exact value."""
+    s = prepare(case, seed)
+    kind = s["kind"]
+    f64 = torch.float64
+    if kind == "linear":
+        m, n, k, w = s["m"], s["n"], s["k"], s["w"]
+        x = _rounded(s["x"], w.dtype, s["gran"])
+        return x @ _decode(w.dtype, w.data, w.sf.buf, 0, n, k, int(w.sf.gran)).t(), None, None
+    if kind == "train":
+        w = s["w"].to(f64)
+        xs, dys = [x.to(f64) for x in s["x"]], [d.to(f64) for d in s["dy"]]
+        return [x @ w.t() for x in xs], [d @ w for d in dys], sum(d.t() @ x for x, d in zip(xs, dys))
+    if kind in ("moe", "moe_ffn"):
+        x, idx, tw = _rounded(s["x"], Dtype.Fp8, 128), s["idx"].long(), s["topk_w"].to(f64)
+        w1 = s["layer"].w if kind == "moe" else s["layer"].w13
+        out = torch.zeros((s["tokens"], s["n"] if kind == "moe" else s["hidden"]), dtype=f64, device=x.device)
+        for e in range(s["experts"]):
+            t, j = (idx == e).nonzero(as_tuple=True)
+            if t.numel() == 0:
+                continue
+            y = x[t] @ _decode(w1.dtype, w1.data, w1.sf.buf, e * w1.rows, w1.rows, w1.k, int(w1.sf.gran)).t()
+            if kind == "moe_ffn":
+                y, w2, i = y.to(torch.bfloat16).to(f64), s["layer"].w2, s["inter"]
+                h = _rounded(y[:, :i] * torch.sigmoid(y[:, :i]) * y[:, i:], Dtype.Fp8, 128)
+                y = h @ _decode(w2.dtype, w2.data, w2.sf.buf, e * w2.rows, w2.rows, w2.k, int(w2.sf.gran)).t()
+            out.index_add_(0, t, y * tw[t, j][:, None])
+        return out
+    if kind == "moe_masked":
+        a, w, mm = s["a"], s["w"], s["max_m"]
+        out = torch.zeros(s["out"].data.shape, dtype=f64, device=s["out"].data.device)
+        for g, r in enumerate(s["masked_m"].tolist()):
+            if r:
+                out[g * mm:g * mm + r] = _decode(a.dtype, a.data, a.sf.buf, g * mm, r, a.k, 128) @ \
+                    _decode(w.dtype, w.data, w.sf.buf, g * w.rows, w.rows, w.k, int(w.sf.gran)).t()
+        return out
+    heads, d, hw = s["heads"], s["dim"], s["hw"].to(f64)
+    logits = torch.zeros(s["logits"].shape, dtype=f64, device=hw.device)
+    if kind == "indexer_paged":
+        dt, per, page, nn = s["q"].dtype, s["per"], s["page"], s["next_n"]
+        kv = _decode(dt, s["kv_pages"], s["kv_words"][None], 0, s["num_pages"] * page, d, 32).view(s["num_pages"], page, d)
+        q = _decode(dt, s["q"].data, s["q"].sf.buf, 0, hw.shape[0] * heads, d, 32).view(-1, heads, d)
+        lens = s["lens"].tolist()
+        for b in range(s["requests"]):
+            rows = kv[s["table"][b * nn, :per].long()].view(per * page, d)
+            for t in range(b * nn, b * nn + nn):
+                logits[t, :lens[t]] = _relu_logits(q[t:t + 1], rows[:lens[t]], hw[t:t + 1])[0]
+        return logits
+    if kind == "indexer":
+        q = s["q"].view(torch.float8_e4m3fn).to(f64)
+        kv = s["kv_codes"].view(torch.float8_e4m3fn).to(f64) * s["scale"].to(f64)[:, None]
+    else:
+        q = _decode(s["q"].dtype, s["q"].data, s["q"].sf.buf, 0, s["tokens"] * heads, d, 32).view(-1, heads, d)
+        kv = _decode(s["kv_op"].dtype, s["kv_op"].data, s["kv_op"].sf.buf, 0, s["kv"], d, 32)
+    ks, ke = s["ks"].tolist(), s["ke"].tolist()
+    for t0 in range(0, s["tokens"], 64):
+        t1 = min(s["tokens"], t0 + 64)
+        lo, hi = min(ks[t0:t1]), max(ke[t0:t1])
+        part = _relu_logits(q[t0:t1], kv[lo:hi], hw[t0:t1])
+        for t in range(t0, t1):
+            logits[t, :ke[t] - ks[t]] = part[t - t0, ks[t] - lo:ke[t] - lo]
+    return logits
