@@ -11,15 +11,16 @@
 
 #include "host.h"
 #include "mx_codec.cuh"
+#include "ptx.cuh"
 
 namespace dg {
 
 
 // ------------------------------------------------------------------------- quant_mx
-// One warp owns 32 consecutive rows x one "span" of 4 scale groups (4*G floats), so that it
-// produces whole SF words: lane r keeps the word of row r and the warp stores 128 contiguous
+// One warp owns R consecutive rows x one "span" of 4 scale groups (4*G floats), so that it
+// produces whole SF words: lane r keeps the word of row r and the warp stores 4*R contiguous
 // bytes of the SF row.  G = 32: one float4 per lane covers the span (8 lanes per group);
-// G = 128: four float4 per lane, load j is group j.
+// G = 128: four float4 per lane, load j is group j.  R is the launcher's choice (eight_rows_per_warp).
 // SWIGLU: the values to quantise are not read as f32 but formed on the fly from the BF16 output
 // [m, 2k] of an MoE gate/up projection (row pitch src_pitch elements): silu(gate) * up with gate =
 // columns [0, k), up = columns [k, 2k), f32 arithmetic on the bf16 values (the golden model's
@@ -29,30 +30,35 @@ namespace dg {
 // (v - lo) / (hi - lo), so that the expectation is v.  The 24 random bits of element (row, col) come from
 // a counter-based hash of its index and `seed`; all the arithmetic is exact in f32, so the result is
 // a pure function of (x, seed) and is checked bit for bit against the same definition on the CPU.
-template <uint32_t G, bool FP4, bool SWIGLU = false, bool STOCH = false, bool PITCHED = false>
+template <uint32_t R, uint32_t G, bool FP4, bool SWIGLU = false, bool STOCH = false, bool PITCHED = false>
 __global__ void __launch_bounds__(256) quant_mx_kernel(const float* __restrict__ x, uint32_t m, uint32_t k,
                                                       uint8_t* __restrict__ data, uint32_t* __restrict__ sf,
                                                       uint32_t sf_cols, uint32_t num_spans, uint32_t num_row_blocks,
-                                                      uint64_t src_pitch = 0, uint32_t seed = 0) {
+                                                      uint64_t src_pitch, uint32_t seed) {
     constexpr uint32_t kLoads = G / 32;                   // float4 loads per lane per row
     // Row pitch of a plain f32 input: K itself unless PITCHED (quantize_output_fp8), as a 32-bit value so that the
     // row offset is one widening multiply.  A run-time 64-bit select in its place made the per-128 kernel 35 %
     // slower (146 against 108 us on 16384 x 7168), a 32-bit one still 7 %.
     const uint32_t x_pitch = PITCHED ? (uint32_t)src_pitch : k;
-    constexpr uint32_t kRowsPerIter = G == 32 ? 8 : 2;    // rows in flight per warp
+    constexpr uint32_t kInFlight = G == 32 ? 8 : 2;       // rows in flight per warp
+    constexpr uint32_t kRowsPerIter = R < kInFlight ? R : kInFlight;
+    static_assert(R <= 32 && R % kRowsPerIter == 0, "a lane keeps the word of one row");
+    // the GEMM behind this kernel sets itself up while the last blocks run; x may come from the kernel before it
+    griddep_wait();
+    griddep_launch_dependents();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp_global = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (warp_global >= num_spans * num_row_blocks) return;
     // Consecutive warps walk the spans of one row block, so a block of 8 warps reads
     // 8 * 4G contiguous floats of each row.
     const uint32_t span = warp_global % num_spans;
-    const uint32_t row0 = (warp_global / num_spans) * 32u;
+    const uint32_t row0 = (warp_global / num_spans) * R;
     const uint32_t num_groups = k / G;
     const uint32_t groups_here = min(4u, num_groups - span * 4u);
     const uint32_t col0 = span * 4u * G;
     uint32_t my_word = 0;
 
-    for (uint32_t rb = 0; rb < 32u; rb += kRowsPerIter) {
+    for (uint32_t rb = 0; rb < R; rb += kRowsPerIter) {
         float4 v[kRowsPerIter][kLoads];
         // SWIGLU: the raw BF16 gate and up values of all rows in flight; every load is issued before the first
         // value is formed (formed inside a branch beside its loads, each pair of loads was waited for in turn
@@ -136,7 +142,7 @@ __global__ void __launch_bounds__(256) quant_mx_kernel(const float* __restrict__
     }
     // One SF word per (span, row); columns m .. sf_cols-1 are padding and get zeros.
     const uint32_t row = row0 + lane;
-    if (row < sf_cols) sf[(size_t)span * sf_cols + row] = my_word;
+    if (lane < R && row < sf_cols) sf[(size_t)span * sf_cols + row] = my_word;
 }
 
 // ------------------------------------------------------------------------- dequant_mx
@@ -230,23 +236,58 @@ static int32_t check_quant_args(const void* x, uint32_t m, uint32_t k, int32_t d
     return DG_OK;
 }
 
+// Rows per warp.  A warp walks its rows a few at a time, each step a trip to memory, so few rows per warp and many
+// warps hide the latency; more rows per warp write longer runs of scale words and, where a row of codes is short (FP4)
+// or a step moves only two rows (per 128), keep more of the reads in a row's run.  Microseconds on B200 with 32 / 8 / 2
+// rows per warp (32, the only choice before, was never the best): per 128, 16 x 7168 21.5 / 6.4 / 2.3, 512 x 7168
+// 27.9 / 8.4 / 4.9, 2019 x 7168 29.7 / 12.8 / 13.5, 16384 x 7168 102 / 93 / 95; per 32, 1021 x 1536 10.7 / 3.2 / 2.6,
+// 16384 x 7168 117 / 110 / 96; FP4, 16 x 16384 5.8 / 2.1 / 1.4, 128 x 7168 6.8 / 2.1 / 2.6, 16384 x 7168 105 / 98 / 117.
+template <uint32_t G, bool FP4>
+static bool eight_rows_per_warp(uint32_t m, uint32_t k) {
+    const uint64_t work = (uint64_t)ceil_div(k / G, 4) * m;      // spans
+    return FP4 ? work >= 4096u : G == 128u && work >= 16384u;
+}
+
+// One quantiser launch: R rows per warp, 8 warps per block; programmatic serialization on both sides (the kernel waits
+// for its predecessor itself and lets its successor set up early).
+template <uint32_t R, uint32_t G, bool FP4, bool SWIGLU, bool STOCH, bool PITCHED>
+static int32_t launch_quant_rows(const void* x, uint32_t m, uint32_t k, void* data_out, uint32_t* sf_out, uint64_t src_pitch,
+                                 uint32_t seed, cudaStream_t s) {
+    const uint32_t sf_cols = align_up(m, 4);
+    const uint32_t num_spans = ceil_div(k / G, 4);
+    const uint32_t num_row_blocks = ceil_div(sf_cols, R);
+    const uint64_t warps = (uint64_t)num_spans * num_row_blocks;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((uint32_t)((warps + 7) / 8));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    DG_CUDA_CHECK(cudaLaunchKernelEx(&cfg, quant_mx_kernel<R, G, FP4, SWIGLU, STOCH, PITCHED>, static_cast<const float*>(x), m, k,
+                                     static_cast<uint8_t*>(data_out), sf_out, sf_cols, num_spans, num_row_blocks, src_pitch, seed));
+    note_launch();
+    return DG_OK;
+}
+
+template <uint32_t G, bool FP4, bool SWIGLU = false, bool STOCH = false, bool PITCHED = false>
+static int32_t launch_quant_kernel(const void* x, uint32_t m, uint32_t k, void* data_out, uint32_t* sf_out, uint64_t src_pitch,
+                                   uint32_t seed, cudaStream_t s) {
+    // SwiGLU forms its values from twice the loads: 2 rows are best at every size (24320 x 2048: 94 / 66 / 62 us)
+    if constexpr (!SWIGLU && !STOCH && !PITCHED && (FP4 || G == 128)) {
+        if (eight_rows_per_warp<G, FP4>(m, k))
+            return launch_quant_rows<8, G, FP4, SWIGLU, STOCH, PITCHED>(x, m, k, data_out, sf_out, src_pitch, seed, s);
+    }
+    return launch_quant_rows<2, G, FP4, SWIGLU, STOCH, PITCHED>(x, m, k, data_out, sf_out, src_pitch, seed, s);
+}
+
 static int32_t launch_quant(const float* x, uint32_t m, uint32_t k, int32_t dtype, uint32_t gran, void* data_out,
                             uint32_t* sf_out, cudaStream_t s) {
-    const uint32_t sf_cols = align_up(m, 4);
-    const uint32_t num_spans = ceil_div(k / gran, 4);
-    const uint32_t num_row_blocks = ceil_div(sf_cols, 32);
-    const uint64_t warps = (uint64_t)num_spans * num_row_blocks;
-    const uint32_t blocks = (uint32_t)((warps + 7) / 8);
-    uint8_t* d = static_cast<uint8_t*>(data_out);
-    if (dtype == DG_FP4)
-        quant_mx_kernel<32, true><<<blocks, 256, 0, s>>>(x, m, k, d, sf_out, sf_cols, num_spans, num_row_blocks);
-    else if (gran == 32)
-        quant_mx_kernel<32, false><<<blocks, 256, 0, s>>>(x, m, k, d, sf_out, sf_cols, num_spans, num_row_blocks);
-    else
-        quant_mx_kernel<128, false><<<blocks, 256, 0, s>>>(x, m, k, d, sf_out, sf_cols, num_spans, num_row_blocks);
-    dg::note_launch();
-    DG_CUDA_CHECK(cudaGetLastError());
-    return DG_OK;
+    if (dtype == DG_FP4) return launch_quant_kernel<32, true>(x, m, k, data_out, sf_out, 0, 0, s);
+    if (gran == 32) return launch_quant_kernel<32, false>(x, m, k, data_out, sf_out, 0, 0, s);
+    return launch_quant_kernel<128, false>(x, m, k, data_out, sf_out, 0, 0, s);
 }
 
 }  // namespace dg
@@ -264,20 +305,9 @@ int32_t dg_swiglu_quant(const void* gate_up_bf16, uint64_t pitch, uint32_t m, ui
     const dg::DeviceInfo* dev;
     int32_t st = dg::current_device(&dev);
     if (st != DG_OK) return st;
-    const uint32_t sf_cols = dg::align_up(m, 4);
-    const uint32_t num_spans = dg::ceil_div(inter / gran, 4);
-    const uint32_t num_row_blocks = dg::ceil_div(sf_cols, 32);
-    const uint32_t blocks = (uint32_t)(((uint64_t)num_spans * num_row_blocks + 7) / 8);
-    const float* src = static_cast<const float*>(gate_up_bf16);
-    uint8_t* d = static_cast<uint8_t*>(data_out);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (gran == 32)
-        dg::quant_mx_kernel<32, false, true><<<blocks, 256, 0, s>>>(src, m, inter, d, sf_out, sf_cols, num_spans, num_row_blocks, pitch);
-    else
-        dg::quant_mx_kernel<128, false, true><<<blocks, 256, 0, s>>>(src, m, inter, d, sf_out, sf_cols, num_spans, num_row_blocks, pitch);
-    dg::note_launch();
-    DG_CUDA_CHECK(cudaGetLastError());
-    return DG_OK;
+    return gran == 32 ? dg::launch_quant_kernel<32, false, true>(gate_up_bf16, m, inter, data_out, sf_out, pitch, 0, s)
+                      : dg::launch_quant_kernel<128, false, true>(gate_up_bf16, m, inter, data_out, sf_out, pitch, 0, s);
 }
 
 int32_t dg_quant_mx(const float* x, uint32_t m, uint32_t k, int32_t dtype, uint32_t gran, void* data_out,
@@ -413,19 +443,9 @@ int32_t dg_quantize_output_fp8(const float* src, uint32_t m, uint32_t n, uint32_
     const dg::DeviceInfo* dev;
     int32_t st = dg::current_device(&dev);
     if (st != DG_OK) return st;
-    const uint32_t sf_cols = dg::align_up(m, 4);
-    const uint32_t num_spans = dg::ceil_div(n / 32, 4);
-    const uint32_t num_row_blocks = dg::ceil_div(sf_cols, 32);
-    const uint32_t blocks = (uint32_t)(((uint64_t)num_spans * num_row_blocks + 7) / 8);
-    uint8_t* d = static_cast<uint8_t*>(data_out);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (stochastic)
-        dg::quant_mx_kernel<32, false, false, true, true><<<blocks, 256, 0, s>>>(src, m, n, d, sf_out, sf_cols, num_spans, num_row_blocks, in_stride, seed);
-    else
-        dg::quant_mx_kernel<32, false, false, false, true><<<blocks, 256, 0, s>>>(src, m, n, d, sf_out, sf_cols, num_spans, num_row_blocks, in_stride);
-    dg::note_launch();
-    DG_CUDA_CHECK(cudaGetLastError());
-    return DG_OK;
+    return stochastic ? dg::launch_quant_kernel<32, false, false, true, true>(src, m, n, data_out, sf_out, in_stride, seed, s)
+                      : dg::launch_quant_kernel<32, false, false, false, true>(src, m, n, data_out, sf_out, in_stride, 0, s);
 }
 
 int32_t dg_transform_sf_host(const float* sf_host, uint32_t mn, uint32_t sf_k, uint32_t* out, void* stream) {

@@ -136,3 +136,15 @@ def test_quant_then_dequant_round_trip_at_full_size():
     same = (sf2.buf == sf.buf).all()
     if bool(same):
         assert torch.equal(data, data2)
+
+
+@pytest.mark.parametrize("m,k,kind,gran", [(2, 16384, "fp8", 128), (511, 16384, "fp8", 128), (512, 16384, "fp8", 128), (2341, 3584, "fp8", 128),
+                                          (31, 16384, "fp4", 32), (32, 16384, "fp4", 32), (4097, 128, "fp4", 32), (263, 7168, "fp8", 32)])
+def test_quant_mx_rows_per_warp(m, k, kind, gran):
+    """Both sides of the lines between two and eight rows per warp, with ragged row counts."""
+    x = _special(m, k, m + k)
+    dt, odt = (Dtype.Fp4, o.FP4) if kind == "fp4" else (Dtype.Fp8, o.FP8)
+    want_data, want_sf = o.quant_mx_host(x, odt, gran)
+    data, sf = quant_mx(dev(x), m, k, dt, gran)
+    torch.cuda.synchronize()
+    assert np.array_equal(sf.buf.cpu().numpy().view(np.uint32), want_sf) and np.array_equal(data.cpu().numpy(), want_data)
