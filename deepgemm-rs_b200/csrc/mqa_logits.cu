@@ -56,6 +56,11 @@ __host__ __device__ constexpr uint32_t mqa_epilogue_regs(uint32_t nun) {
 }
 static_assert(mqa_launch_regs(4) == 96 && mqa_epilogue_regs(4) == 104, "register budget of the 64-head variant");
 static_assert(mqa_launch_regs(8) == 168 && mqa_epilogue_regs(8) == 232, "register budget of the 128-head variant");
+constexpr uint32_t kDecStages = 6;         // decode: accumulator stages at most
+constexpr uint32_t kDecAccCols = 384;      // decode: columns they share
+constexpr uint32_t kDecArrivals = 48;      // decode: arrivals that free a stage, split evenly over its 4 nq reducing warps (nq <= 4)
+__host__ __device__ constexpr uint32_t dec_block_q(uint32_t heads) { return heads == 64 ? 3u : 4u; }   // queries of a request per task
+constexpr uint32_t kPagesAhead = 8;        // paged: block-table look-ups run so many kv blocks ahead
 constexpr uint32_t kMqaSfaCol = 448;       // ue8m0 contracts only: the accumulators are <= 192 wide
 constexpr uint32_t kMqaSfbCol = 452;
 
@@ -98,7 +103,7 @@ struct __align__(8) MqaBarriers {
     uint64_t kv_ready[kMqaMaxKvStages];   // ue8m0: scale factors in place
     uint64_t kv_empty[kMqaMaxKvStages];
     uint64_t q_full[2], q_ready[2], q_empty[2];
-    uint64_t tmem_full[2], tmem_empty[2];
+    uint64_t tmem_full[kDecStages], tmem_empty[kDecStages];   // two of them outside decode
     uint64_t w_full[2];                   // weights of a task staged by the epilogue warps
     uint32_t tmem_base;
     uint32_t abort;
@@ -220,9 +225,13 @@ __device__ __forceinline__ float relu_nan(float x) {
 // U4: head counts that are not a multiple of 16 (their 4-column reduction loop is a variant of its own: as a
 // run-time branch beside the 16-column loop it cost the common case 4 %).
 // QPW: queries per warpgroup of the NUN variants (their NUN units are QPW queries of 16 * NUN / QPW heads).
+// DEC (paged, 32 or 64 heads): decode.  A request has one to four tokens, so with one warpgroup per query of the block
+// most warpgroups had nothing to reduce and the live ones ran at the latency of their TMEM loads.  Here the four
+// warpgroups take (query, kv block) pairs: with nq queries in a task, 4 / nq kv blocks are reduced side by side, the
+// MMAs are only nq queries wide and the accumulator ring has as many stages as then fit in kDecAccCols columns.
 // NUN: 16-column units a warpgroup reduces per kv block when that is known at compile time (4 / 8 = one query of
 // 64 / 128 heads per warpgroup: the unit loop is then straight-line code without counters), 0 = any.
-template <bool SCALED, bool FP4, bool PAGED, bool U4 = false, uint32_t NUN = 0, uint32_t QPW = 1>
+template <bool SCALED, bool FP4, bool PAGED, bool U4 = false, uint32_t NUN = 0, uint32_t QPW = 1, bool DEC = false>
 __global__ void __launch_bounds__(mqa_threads(NUN), 1)
 mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
                   const __grid_constant__ CUtensorMap tm_qsf, const __grid_constant__ CUtensorMap tm_kvsf,
@@ -243,7 +252,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         bars->abort = 0;
         for (uint32_t s = 0; s < p.kv_stages; ++s) {
             mbar_init(smem_u32(&bars->kv_full[s]), 1);
-            mbar_init(smem_u32(&bars->kv_ready[s]), 1);
+            mbar_init(smem_u32(&bars->kv_ready[s]), PAGED ? 32 : 1);   // paged: one arrival per lane of the SF warp
             mbar_init(smem_u32(&bars->kv_empty[s]), 1);
         }
         for (uint32_t s = 0; s < 2; ++s) {
@@ -251,8 +260,10 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             mbar_init(smem_u32(&bars->q_ready[s]), 1);
             mbar_init(smem_u32(&bars->q_empty[s]), 1);
             mbar_init(smem_u32(&bars->w_full[s]), ep_warps);
+        }
+        for (uint32_t s = 0; s < (DEC ? kDecStages : 2u); ++s) {
             mbar_init(smem_u32(&bars->tmem_full[s]), 1);
-            mbar_init(smem_u32(&bars->tmem_empty[s]), ep_warps);
+            mbar_init(smem_u32(&bars->tmem_empty[s]), DEC ? kDecArrivals : ep_warps);
         }
         fence_barrier_init();
         tma_prefetch_desc(&tm_q);
@@ -294,8 +305,8 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             __syncwarp();
             if (PAGED) {
                 // A block of 128 tokens is a run of whole pages (or half / a quarter of a large page): lane i looks up
-                // the page of box i in the block table.  The look-ups run four blocks ahead of the loads, and the
-                // loop is unrolled by four so that an entry stays in its register, untouched, until its block comes
+                // the page of box i in the block table.  The look-ups run eight blocks ahead of the loads, and the
+                // loop is unrolled so that an entry stays in its register, untouched, until its block comes
                 // up: looked up inside the loop, each block cost the producer a trip to memory, and decode ran at
                 // that latency instead of the cache's bandwidth.
                 const uint32_t* trow = p.block_table + (size_t)k.table_row * p.block_table_stride;
@@ -305,13 +316,13 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     const uint32_t pg = tok_of(kbx) >> page_shift;
                     return (kbx < k.kb1 && lane < p.boxes_per_block && pg < p.block_table_stride) ? __ldg(trow + pg) : 0u;
                 };
-                uint32_t pq[4];
+                uint32_t pq[kPagesAhead];
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) pq[j] = page_of(k.kb0 + j);
-                for (uint32_t kb4 = k.kb0; ok && kb4 < k.kb1; kb4 += 4u) {
+                for (uint32_t j = 0; j < kPagesAhead; ++j) pq[j] = page_of(k.kb0 + j);
+                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kPagesAhead) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j) {
-                        const uint32_t kb = kb4 + j;
+                    for (uint32_t j = 0; j < kPagesAhead; ++j) {
+                        const uint32_t kb = kb0 + j;
                         if (kb >= k.kb1) break;
                         if (!(ok = DG_WARP_WAIT(smem_u32(&bars->kv_empty[stage]), phase ^ 1u, wc, kWaitEmpty))) break;
                         const uint32_t bar = smem_u32(&bars->kv_full[stage]);
@@ -319,7 +330,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         // rows past the table's width or pages outside the cache read row 0 (paged_row)
                         uint32_t row = pq[j] * p.page_kv + (tok_of(kb) & (p.page_kv - 1u));
                         if (row + p.box_rows > p.num_kv) row = 0u;
-                        pq[j] = page_of(kb + 4u);
+                        pq[j] = page_of(kb + kPagesAhead);
                         if (lane == 0) mbar_arrive_expect_tx(bar, kv_tx);
                         __syncwarp();
                         if (lane < p.boxes_per_block) tma_load_2d(&tm_kv, bar, dst + lane * p.box_rows * p.row_bytes, 0, (int32_t)row);
@@ -345,6 +356,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     } else if (warp == 1) {
         // ===================================================== MMA issuer (warp-converged, one lane issues)
         uint32_t stage = 0, phase = 0, qcount = 0, acount = 0;
+        uint32_t acc_bits = 0;      // DEC: per accumulator stage, parity of its uses so far
         bool ok = true;
         MqaTasks<PAGED> tasks(p);
         MqaTask k;
@@ -368,16 +380,29 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 return kLaneLoop ? mbar_wait(bar, parity, wc, site) : (bool)DG_WARP_WAIT(bar, parity, wc, site);
             };
             if (!kLaneLoop || issuer) {
+            // DEC: width and number of the accumulator stages of this task; the ring starts over at its first stage once
+            // every stage of the task before (of another width, maybe) has been drained
+            const uint32_t dec_width = k.nq * p.num_heads, dec_stages = DEC ? min(kDecStages, kDecAccCols / dec_width) : 0u;
+            const uint32_t idesc = DEC ? make_idesc_bs(FP4 ? 1u : 0u, FP4 ? 1u : 0u, kMqaBlockKv, dec_width) : p.idesc;
+            uint32_t ring = 0;
+            if (DEC)
+                for (uint32_t s = 0; ok && s < kDecStages; ++s)
+                    ok = wait_on(smem_u32(&bars->tmem_empty[s]), ((acc_bits >> s) & 1u) ^ 1u, kWaitTmemEmpty);
             for (uint32_t kb = k.kb0; ok && kb < k.kb1; ++kb) {
                 if (!(ok = wait_on(smem_u32(&bars->kv_full[stage]), phase, kWaitFull))) break;
                 if (SCALED && !(ok = wait_on(smem_u32(&bars->kv_ready[stage]), phase, kWaitSfReady))) break;
+                if (PAGED) fence_proxy_async_smem();     // the scale words came by generic-proxy copies, tcgen05.cp reads them
                 const uint32_t kaddr = base + p.off_kv + stage * p.kv_stage_bytes;
                 const uint64_t kv_desc = make_smem_desc(kaddr, p.sbo, 0, p.layout);
-                const uint32_t as = acount & 1u, aphase = (acount >> 1) & 1u;
+                const uint32_t as = DEC ? ring : acount & 1u, aphase = DEC ? (acc_bits >> ring) & 1u : (acount >> 1) & 1u;
                 ++acount;
+                if (DEC) {
+                    acc_bits ^= 1u << ring;
+                    if (++ring == dec_stages) ring = 0;
+                }
                 if (!(ok = wait_on(smem_u32(&bars->tmem_empty[as]), aphase ^ 1u, kWaitTmemEmpty))) break;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem + as * acc_stride;
+                const uint32_t d_tmem = tmem + as * (DEC ? dec_width : acc_stride);
                 if (kLaneLoop || elect_one()) {
                     if (SCALED) {
                         if (!q_sf_copied)    // the q scales of this task: in order behind every MMA that used the previous task's
@@ -387,13 +412,13 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     }
                     for (uint32_t m = 0; m < p.num_mma; ++m) {
                         if (SCALED && FP4)      // 64 elements per MMA: half-word (m & 1) of the row's scale word
-                            tc_mma_mxf4(d_tmem, kv_desc + 2u * m, q_desc + 2u * m, idesc_with_sf_ids(p.idesc, (m & 1u) * 2u, (m & 1u) * 2u),
+                            tc_mma_mxf4(d_tmem, kv_desc + 2u * m, q_desc + 2u * m, idesc_with_sf_ids(idesc, (m & 1u) * 2u, (m & 1u) * 2u),
                                         m != 0u, tmem + kMqaSfaCol, tmem + kMqaSfbCol);
                         else if (SCALED)
-                            tc_mma_mxf8(d_tmem, kv_desc + 2u * m, q_desc + 2u * m, idesc_with_sf_ids(p.idesc, m, m), m != 0u,
+                            tc_mma_mxf8(d_tmem, kv_desc + 2u * m, q_desc + 2u * m, idesc_with_sf_ids(idesc, m, m), m != 0u,
                                         tmem + kMqaSfaCol, tmem + kMqaSfbCol);
                         else
-                            tc_mma_f8(d_tmem, kv_desc + 2u * m, q_desc + 2u * m, p.idesc, m != 0u);
+                            tc_mma_f8(d_tmem, kv_desc + 2u * m, q_desc + 2u * m, idesc, m != 0u);
                     }
                     tc_commit(smem_u32(&bars->kv_empty[stage]));
                     tc_commit(smem_u32(&bars->tmem_full[as]));
@@ -410,6 +435,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 stage = __shfl_sync(0xffffffffu, stage, issuer_lane);
                 phase = __shfl_sync(0xffffffffu, phase, issuer_lane);
                 acount = __shfl_sync(0xffffffffu, acount, issuer_lane);
+                acc_bits = __shfl_sync(0xffffffffu, acc_bits, issuer_lane);
                 ok = __shfl_sync(0xffffffffu, (uint32_t)ok, issuer_lane) != 0u;
             }
         }
@@ -440,47 +466,35 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             if (lane == 0) mbar_arrive(smem_u32(&bars->q_ready[qs]));
             if (PAGED) {
                 // Lane l fetches the words of tokens 4 l .. 4 l + 3 of a block: they lie in one page (pages hold a
-                // multiple of four tokens), so it is one block-table entry and one 16-byte load.  Both run ahead
-                // of the block that is written -- entries four blocks, words two -- in registers that are not touched
-                // before their block comes up (the loop is unrolled by four for that): fetched inside the loop, one
-                // after the other, they cost two trips to memory per block, and decode ran at that latency.
+                // multiple of four tokens), so it is one block-table entry.  The words are copied asynchronously, straight
+                // to their places in the stage, and the stage's barrier counts the lanes' copies: as many blocks are under
+                // way as the ring has stages.  (Held in registers two blocks ahead, a load's trip to memory every two
+                // blocks bounded decode: 690 ns per block.)  The block-table entries run eight blocks ahead in
+                // registers that are not touched before their block comes up; the loop is unrolled for that.
                 const uint32_t* trow = p.block_table + (size_t)k.table_row * p.block_table_stride;
                 const uint32_t page_shift = (uint32_t)__ffs((int)p.page_kv) - 1u;
                 auto page_of = [&](uint32_t kbx) -> uint32_t {
                     const uint32_t pg = (kbx * kMqaBlockKv + 4u * lane) >> page_shift;
                     return (kbx < k.kb1 && pg < p.block_table_stride) ? __ldg(trow + pg) : 0u;
                 };
-                auto words_of = [&](uint32_t kbx, uint32_t page) -> uint4 {
-                    uint32_t row = page * p.page_kv + ((kbx * kMqaBlockKv + 4u * lane) & (p.page_kv - 1u));
-                    if (row + 4u > p.num_kv) row = 0u;       // tokens past the table or the cache: masked by the epilogue
-                    return __ldg(reinterpret_cast<const uint4*>(p.kv_sf + row));
-                };
-                uint32_t pq[4];
-                uint4 wq2[2];
+                uint32_t pq[kPagesAhead];
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) pq[j] = page_of(k.kb0 + j);
-                wq2[0] = words_of(k.kb0, pq[0]);
-                wq2[1] = words_of(k.kb0 + 1u, pq[1]);
-                for (uint32_t kb4 = k.kb0; ok && kb4 < k.kb1; kb4 += 4u) {
+                for (uint32_t j = 0; j < kPagesAhead; ++j) pq[j] = page_of(k.kb0 + j);
+                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kPagesAhead) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j) {
-                        const uint32_t kb = kb4 + j;
+                    for (uint32_t j = 0; j < kPagesAhead; ++j) {
+                        const uint32_t kb = kb0 + j;
                         if (kb >= k.kb1) break;
-                        const uint4 cur = wq2[j & 1u];
-                        wq2[j & 1u] = words_of(kb + 2u, pq[(j + 2u) & 3u]);
-                        pq[j] = page_of(kb + 4u);
                         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->kv_empty[stage]), phase ^ 1u, wc, kWaitEmpty));
                         if (!ok) break;
-                        uint32_t* sf = reinterpret_cast<uint32_t*>(base_ptr + p.off_kv + stage * p.kv_stage_bytes + p.kv_sf_off);
+                        uint32_t row = pq[j] * p.page_kv + ((kb * kMqaBlockKv + 4u * lane) & (p.page_kv - 1u));
+                        if (row + 4u > p.num_kv) row = 0u;       // tokens past the table or the cache: masked by the epilogue
+                        pq[j] = page_of(kb + kPagesAhead);
                         // row r = 4 l + i of the block goes to position 4 (r % 32) + r / 32
-                        const uint32_t hi = lane >> 3;
-                        sf[4u * ((4u * lane + 0u) & 31u) + hi] = cur.x;
-                        sf[4u * ((4u * lane + 1u) & 31u) + hi] = cur.y;
-                        sf[4u * ((4u * lane + 2u) & 31u) + hi] = cur.z;
-                        sf[4u * ((4u * lane + 3u) & 31u) + hi] = cur.w;
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&bars->kv_ready[stage]));
+                        const uint32_t sf = base + p.off_kv + stage * p.kv_stage_bytes + p.kv_sf_off + (lane >> 3) * 4u;
+#pragma unroll
+                        for (uint32_t i = 0; i < 4; ++i) cp_async_4(sf + 16u * ((4u * lane + i) & 31u), p.kv_sf + row + i);
+                        cp_async_arrive(smem_u32(&bars->kv_ready[stage]));
                         if (++stage == p.kv_stages) { stage = 0; phase ^= 1u; }
                     }
                 }
@@ -502,11 +516,11 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
     } else {
         // ===================================================== epilogue warpgroups
-        if (NUN) reg_acquire<mqa_epilogue_regs(NUN)>();
+        if (NUN) reg_acquire<mqa_epilogue_regs(NUN == 2u ? 4u : NUN)>();
         const uint32_t et = threadIdx.x - 128u;
         const uint32_t wg = et >> 7;                  // warpgroup index
         const uint32_t quarter = warp & 3u;           // TMEM lane quarter of this warp
-        uint32_t qcount = 0, acount = 0;
+        uint32_t qcount = 0, acount = 0, acc_bits = 0;
         bool ok = true;
         MqaTasks<PAGED> tasks(p);
         MqaTask k;
@@ -558,6 +572,60 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 if (lane == 0) mbar_arrive(smem_u32(&bars->w_full[wb]));
                 ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->w_full[wb]), wphase, wc, kWaitWeights));
                 if (!ok) break;
+                if (DEC) {
+                    // This warpgroup reduces query qi of every kv block with index = group (mod groups).  The ring of
+                    // accumulator stages is walked over all kv blocks; a stage's barrier cannot be a use behind when it
+                    // is waited on, because the ring has at least as many stages as there are groups, the commits
+                    // complete in order, and no warp enters a task (w_full) before all have left the one before.
+                    const uint32_t groups = 4u / k.nq, group = wg / k.nq, qi = wg - group * k.nq;
+                    const uint32_t width = k.nq * p.num_heads, stages = min(kDecStages, kDecAccCols / width);
+                    const uint32_t blocks = k.kb1 - k.kb0, share = kDecArrivals / (4u * k.nq);
+                    const uint32_t s_fix = win[qi], e_fix = win[16u + qi];
+                    const uint32_t span = e_fix > s_fix ? e_fix - s_fix : 0u;
+                    __nv_bfloat16* const out = reinterpret_cast<__nv_bfloat16*>(p.logits) + (size_t)(k.q0 + qi) * p.logits_stride;
+                    const uint32_t lane_base = tmem + ((quarter * 32u) << 16) + qi * 16u * NUN;
+                    uint64_t wp[NUN ? 8u * NUN : 1u];
+#pragma unroll
+                    for (uint32_t i = 0; i < 4u * NUN; ++i) {
+                        const float4 w4 = reinterpret_cast<const float4*>(w + qi * 16u * NUN)[i];
+                        wp[2 * i] = pack_f32x2(w4.x, w4.y);
+                        wp[2 * i + 1] = pack_f32x2(w4.z, w4.w);
+                    }
+                    uint32_t as = 0, turn = 0;               // stage and (block index mod groups) of the current kv block
+                    for (uint32_t b = 0; b < blocks; ++b) {
+                        const uint32_t aphase = (acc_bits >> as) & 1u, cur = as;
+                        const bool mine = turn == group;
+                        acc_bits ^= 1u << as;
+                        if (++as == stages) as = 0;
+                        if (++turn == groups) turn = 0;
+                        if (!mine) continue;
+                        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->tmem_full[cur]), aphase, wc, kWaitTmemFull));
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t taddr = lane_base + cur * width;
+                        uint64_t a01 = 0ull, a23 = 0ull;
+                        uint32_t v[16];
+#pragma unroll
+                        for (uint32_t u = 0; u < NUN; ++u) {
+                            tmem_ld_x16(taddr + u * 16u, v);
+                            tmem_ld_wait();
+                            if (u + 1 == NUN) {
+                                tc_fence_before();
+                                if (lane == 0) mbar_arrive_n(smem_u32(&bars->tmem_empty[cur]), share);
+                            }
+#pragma unroll
+                            for (uint32_t i = 0; i < 4; ++i) {
+                                const float x0 = __uint_as_float(v[4 * i]), x1 = __uint_as_float(v[4 * i + 1]);
+                                const float x2 = __uint_as_float(v[4 * i + 2]), x3 = __uint_as_float(v[4 * i + 3]);
+                                a01 = fma_f32x2(pack_f32x2(relu_nan(x0), relu_nan(x1)), wp[8 * u + 2 * i], a01);
+                                a23 = fma_f32x2(pack_f32x2(relu_nan(x2), relu_nan(x3)), wp[8 * u + 2 * i + 1], a23);
+                            }
+                        }
+                        const uint32_t off = (k.kb0 + b) * kMqaBlockKv + quarter * 32u + lane - s_fix;
+                        if (off < span) out[off] = __float2bfloat16_rn((lo_f32(a01) + hi_f32(a01)) + (lo_f32(a23) + hi_f32(a23)));
+                    }
+                    continue;
+                }
                 if (NUN) {
                     // QPW queries of 16 * NUN / QPW heads per warpgroup, NUN 16-column units per kv block.  The
                     // weights do not change over the kv blocks of the task: they are read from shared memory once,
@@ -583,21 +651,6 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         wp[2 * i + 1] = pack_f32x2(w4.z, w4.w);
                     }
                     uint32_t j = k.kb0 * kMqaBlockKv + quarter * 32u + lane;
-                    // A warpgroup none of whose queries the task has (decode: one or two tokens of a request in a block
-                    // of three or four) only hands the accumulator stages back; its issue slots go to the others.
-                    // (A loop of its own: as a branch inside the reduction loop below it cost that loop 17 %.)
-                    if (PAGED && q_first >= k.nq) {
-                        for (uint32_t kb = k.kb0; kb < k.kb1; ++kb) {
-                            const uint32_t as = acount & 1u, aphase = (acount >> 1) & 1u;
-                            ++acount;
-                            ok = __all_sync(0xffffffffu, mbar_wait(full0 + as * 8u, aphase, wc, kWaitTmemFull));
-                            if (!ok) break;
-                            tc_fence_after();
-                            tc_fence_before();
-                            if (lane == 0) mbar_arrive(empty0 + as * 8u);
-                        }
-                        continue;
-                    }
                     for (uint32_t kb = k.kb0; kb < k.kb1; ++kb, j += kMqaBlockKv) {
                         const uint32_t as = acount & 1u, aphase = (acount >> 1) & 1u;
                         ++acount;
@@ -746,33 +799,45 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 // A query block needs the kv tokens [0, context length of its last token): context lengths grow inside a
 // request (deepgemm/kernels/mqa_logits_sm100.cu:207-216), so that is the longest of its own.
 constexpr uint32_t kMetaThreads = 1024;
-__device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t* sh, bool use_max) {
-    // exclusive scan (sum or max) of one value per thread over the block; identity 0
-    const uint32_t tid = threadIdx.x;
-    sh[tid] = v;
+// Exclusive scan (sum or max) of one value per thread over the block, identity 0: inside the warps by shuffles, then
+// over the 32 warp totals.  sh: 32 words.
+template <bool MAX>
+__device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t* sh) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    auto warp_scan = [&](uint32_t x) {
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x = MAX ? max(x, o) : x + o;
+        }
+        return x;
+    };
+    const uint32_t incl = warp_scan(v);
+    if (lane == 31) sh[warp] = incl;
     __syncthreads();
-    for (uint32_t d = 1; d < kMetaThreads; d <<= 1) {
-        const uint32_t other = tid >= d ? sh[tid - d] : 0u;
-        __syncthreads();
-        sh[tid] = use_max ? max(sh[tid], other) : sh[tid] + other;
-        __syncthreads();
-    }
-    const uint32_t r = tid ? sh[tid - 1] : 0u;
+    if (warp == 0) sh[lane] = warp_scan(sh[lane]);
     __syncthreads();
-    return r;
+    const uint32_t before = warp ? sh[warp - 1u] : 0u;
+    uint32_t prev = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) prev = 0u;
+    __syncthreads();
+    return MAX ? max(before, prev) : before + prev;
 }
 __global__ void __launch_bounds__(kMetaThreads) mqa_paged_metadata_kernel(const uint32_t* __restrict__ context_lens,
                                                                          const uint32_t* __restrict__ indices, uint32_t num_tokens,
                                                                          uint32_t block_q, uint32_t max_ctx, uint32_t* cum,
                                                                          uint32_t* qb_tokens, uint32_t* req_first) {
-    __shared__ uint32_t sh[kMetaThreads];
+    static_assert(kMetaThreads == 1024, "32 warp totals");
+    __shared__ uint32_t sh[32];
+    griddep_wait();
+    griddep_launch_dependents();
     const uint32_t per = (num_tokens + kMetaThreads - 1) / kMetaThreads;
     const uint32_t t0 = min(threadIdx.x * per, num_tokens), t1 = min(t0 + per, num_tokens);
     // request starts: running maximum of (start position + 1)
     uint32_t run = 0;
     for (uint32_t t = t0; t < t1; ++t)
         if (t == 0 || indices[t] != indices[t - 1]) run = t + 1;
-    uint32_t carry = block_scan_excl(run, sh, true);
+    uint32_t carry = block_scan_excl<true>(run, sh);
     for (uint32_t t = t0; t < t1; ++t) {
         if (t == 0 || indices[t] != indices[t - 1]) carry = t + 1;
         req_first[t] = carry - 1u;
@@ -789,7 +854,7 @@ __global__ void __launch_bounds__(kMetaThreads) mqa_paged_metadata_kernel(const 
         qb_tokens[t] = nq;
         if (nq) local += (min(context_lens[t + nq - 1], max_ctx) + kMqaBlockKv - 1) / kMqaBlockKv;
     }
-    uint32_t acc = block_scan_excl(local, sh, false);
+    uint32_t acc = block_scan_excl<false>(local, sh);
     for (uint32_t t = t0; t < t1; ++t) {
         cum[t] = acc;
         const uint32_t nq = qb_tokens[t];
@@ -840,7 +905,10 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
     // columns of the ue8m0 contracts keep all three (six) queries that fit, on three warpgroups (one query of 64
     // heads or two of 32 each): with two queries the MMAs are 128 columns wide and only eight warps reduce.
     const bool three_groups = SCALED && ((num_heads == 64 && block_q == 3) || (num_heads == 32 && block_q == 6));
-    if (three_groups) { /* keep */ }
+    // decode: one to four tokens of a request, four warpgroups over (query, kv block) pairs
+    const bool dec = PAGED && (num_heads == 64 || num_heads == 32);
+    if (dec) block_q = dec_block_q(num_heads);
+    else if (three_groups) { /* keep */ }
     else if (block_q >= 4) block_q &= ~3u;
     else if (block_q == 3) block_q = 2;
     if (block_q == 0) return fail(DG_ERR_UNSUPPORTED, "mqa_logits: %u heads do not fit the %u score columns of this contract", num_heads, max_n);
@@ -848,7 +916,7 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
     p.block_q = block_q;
     p.n = block_q * num_heads;
     p.n_mma = align_up(p.n, 16);
-    p.ep_groups = three_groups ? 3u : block_q % 4 == 0 ? 4u : block_q % 2 == 0 ? 2u : 1u;
+    p.ep_groups = dec ? 4u : three_groups ? 3u : block_q % 4 == 0 ? 4u : block_q % 2 == 0 ? 2u : 1u;
     p.unit = num_heads % 16 == 0 ? 16u : 4u;
     p.num_q_blocks = ceil_div(num_tokens, block_q);
     // Contiguous kv: the work items are query blocks, each over its whole kv range.  With fewer query blocks than
@@ -934,9 +1002,22 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
         uint32_t* req_first = qb_tokens + num_tokens;
         p.cum = cum; p.qb_tokens = qb_tokens; p.req_first = req_first;
         const uint64_t max_ctx64 = (uint64_t)pg.block_table_stride * pg.page_kv;
-        mqa_paged_metadata_kernel<<<1, kMetaThreads, 0, s>>>(pg.context_lens, pg.indices, num_tokens, block_q,
-                                                             (uint32_t)(max_ctx64 > 0xffffff00ull ? 0xffffff00ull : max_ctx64), cum,
-                                                             qb_tokens, req_first);
+        cudaLaunchConfig_t mcfg = {};
+        mcfg.gridDim = dim3(1);
+        mcfg.blockDim = dim3(kMetaThreads);
+        mcfg.stream = s;
+        cudaLaunchAttribute mattr[1];
+        mattr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        mattr[0].val.programmaticStreamSerializationAllowed = 1;
+        mcfg.attrs = mattr;
+        mcfg.numAttrs = 1;
+        const cudaError_t me = cudaLaunchKernelEx(&mcfg, mqa_paged_metadata_kernel, pg.context_lens, pg.indices, num_tokens, block_q,
+                                                  (uint32_t)(max_ctx64 > 0xffffff00ull ? 0xffffff00ull : max_ctx64), cum, qb_tokens,
+                                                  req_first);
+        if (me != cudaSuccess) {
+            if (meta_owned) cudaFreeAsync(meta, s);
+            return fail(DG_ERR_DRIVER, "mqa_logits metadata launch failed: %s", cudaGetErrorString(me));
+        }
         note_launch();
     }
 
@@ -1000,30 +1081,30 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
         const uint32_t threads = cfg.blockDim.x;
         return threads <= mqa_threads(nun) && regs * threads >= 128u * kMqaRoleRegs + (threads - 128u) * mqa_epilogue_regs(nun);
     };
-    if (p.unit == 4u) {
-        auto* fn = mqa_logits_kernel<SCALED, FP4, PAGED, true>;
+    bool fits = true;
+    auto run = [&](auto* fn, uint32_t nun) {      // nun != 0: a kernel that moves registers between its warpgroups
+        fits = nun == 0u || budget_ok((const void*)fn, nun);
+        if (!fits) return;
         e = set_smem((const void*)fn);
         if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fn, tq, tkv, tqsf, tkvsf, p);
-    } else if (num_heads == 32 && p.block_q == 2u * p.ep_groups && p.ep_groups >= 3u) {
-        auto* fn = mqa_logits_kernel<SCALED, FP4, PAGED, false, 4, 2>;   // two queries of 32 heads per warpgroup
-        if (!budget_ok((const void*)fn, 4)) return fail_free(fail(DG_ERR_RUNTIME, "mqa_logits: register budget of the 32-head kernel does not add up"));
-        e = set_smem((const void*)fn);
-        if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fn, tq, tkv, tqsf, tkvsf, p);
-    } else if (num_heads == 64 && p.block_q == p.ep_groups) {
-        auto* fn = mqa_logits_kernel<SCALED, FP4, PAGED, false, 4>;   // one query of 64 heads per warpgroup
-        if (!budget_ok((const void*)fn, 4)) return fail_free(fail(DG_ERR_RUNTIME, "mqa_logits: register budget of the 64-head kernel does not add up"));
-        e = set_smem((const void*)fn);
-        if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fn, tq, tkv, tqsf, tkvsf, p);
-    } else if (num_heads == 128 && p.block_q == p.ep_groups) {
-        auto* fn = mqa_logits_kernel<SCALED, FP4, PAGED, false, 8>;   // one query of 128 heads per warpgroup
-        if (!budget_ok((const void*)fn, 8)) return fail_free(fail(DG_ERR_RUNTIME, "mqa_logits: register budget of the 128-head kernel does not add up"));
-        e = set_smem((const void*)fn);
-        if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fn, tq, tkv, tqsf, tkvsf, p);
+    };
+    e = cudaSuccess;
+    bool done = false;
+    if constexpr (PAGED) {
+        done = dec;
+        if (dec && num_heads == 64) run(mqa_logits_kernel<SCALED, FP4, true, false, 4, 1, true>, 4);
+        else if (dec) run(mqa_logits_kernel<SCALED, FP4, true, false, 2, 1, true>, 4);
     } else {
-        auto* fn = mqa_logits_kernel<SCALED, FP4, PAGED, false>;
-        e = set_smem((const void*)fn);
-        if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fn, tq, tkv, tqsf, tkvsf, p);
+        done = (num_heads == 32 && p.block_q == 2u * p.ep_groups && p.ep_groups >= 3u) || (num_heads == 64 && p.block_q == p.ep_groups);
+        if (done && num_heads == 32) run(mqa_logits_kernel<SCALED, FP4, false, false, 4, 2>, 4);     // two queries of 32 heads per warpgroup
+        else if (done) run(mqa_logits_kernel<SCALED, FP4, false, false, 4>, 4);                      // one query of 64 heads per warpgroup
     }
+    if (!done) {
+        if (p.unit == 4u) run(mqa_logits_kernel<SCALED, FP4, PAGED, true>, 0);
+        else if (num_heads == 128 && p.block_q == p.ep_groups) run(mqa_logits_kernel<SCALED, FP4, PAGED, false, 8>, 8);   // one query of 128 heads per warpgroup
+        else run(mqa_logits_kernel<SCALED, FP4, PAGED, false>, 0);
+    }
+    if (!fits) return fail_free(fail(DG_ERR_RUNTIME, "mqa_logits: register budget of the %u-head kernel does not add up", num_heads));
     if (meta_owned) cudaFreeAsync(meta, s);
     if (e != cudaSuccess) return fail(DG_ERR_DRIVER, "mqa_logits launch failed: %s", cudaGetErrorString(e));
     dg::note_launch();

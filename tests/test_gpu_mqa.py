@@ -184,3 +184,54 @@ def test_mqa_logits_paged(kind, H, D, page_kv):
             assert (got[t0:t0 + n] == fill).all()
             continue
         _check(got[t0:t0 + n], o.bf16_bits_to_f32(o.f32_to_bf16_bits_np(ref)), ks, ke, width, fill)
+
+
+@pytest.mark.parametrize("kind,H,page_kv", [("fp8", 64, 16), ("fp8", 32, 64), ("fp4", 64, 32)])
+def test_mqa_logits_paged_many_requests(kind, H, page_kv):
+    """More requests than SMs, one to six tokens each in random order, so that every CTA walks several tasks whose
+    accumulator rings differ in width and whose kv ranges begin inside a request."""
+    from deepgemm import mqa_logits_paged
+    rng = np.random.default_rng(H + page_kv)
+    D, odt, dt = 128, *((o.FP8, Dtype.Fp8) if kind == "fp8" else (o.FP4, Dtype.Fp4))
+    nreq = 400
+    ntok, last = rng.integers(1, 7, nreq), rng.integers(0, 900, nreq)
+    T, per = int(ntok.sum()), -(-900 // page_kv)
+    num_pages = nreq * per
+    kvf = randn((num_pages * page_kv, D), 3)
+    codes, words = o.quant_mx_host(kvf, odt, 32)
+    kvd = o.dequant_mx_host(codes, words, num_pages * page_kv, D, odt, 32).reshape(num_pages, page_kv, D)
+    perm = rng.permutation(num_pages).astype(np.int32).reshape(nreq, per)
+    first = np.concatenate([[0], np.cumsum(ntok)[:-1]])
+    table = np.full((T, per), 10 ** 6, dtype=np.int32)
+    table[first] = perm
+    indices = np.repeat(np.arange(nreq, dtype=np.int32) * 3 + 1, ntok)
+    ctx = np.concatenate([np.maximum(0, c - (n - 1 - np.arange(n))) for n, c in zip(ntok, last)]).astype(np.int32)
+    qf = randn((T * H, D), 5)
+    qc, qsf = o.quant_mx_host(qf, odt, 32)
+    qd = o.dequant_mx_host(qc, qsf, T * H, D, odt, 32).reshape(T, H, D)
+    wb = torch.from_numpy(randn((T, H), 6)).to(torch.bfloat16)
+    width, fill = 904, -5.0
+    logits = torch.full((T, width), fill, dtype=torch.bfloat16, device="cuda")
+    qop = Operand.k_major(dt, T * H, D, D, sf_tensor(qsf, 32), dev(qc))
+    mqa_logits_paged(qop, dev(codes), dev(words[0, :num_pages * page_kv].view(np.int32)), wb.cuda(), page_kv, num_pages, dev(ctx),
+                     dev(indices), dev(table), per, T, H, D, logits, width)
+    poll_device_status()
+    got = logits.float().cpu().numpy()
+    for r in range(0, nreq, 7):
+        rows = slice(first[r], first[r] + ntok[r])
+        c = ctx[rows]
+        assert all((got[t, n:] == fill).all() for t, n in zip(range(rows.start, rows.stop), c))
+        if c.max() == 0:
+            continue
+        kv = kvd[perm[r]].reshape(-1, D)[:c.max()]
+        ref = o.mqa_logits_ref(qd[rows], kv, wb.float().numpy()[rows], np.zeros(len(c), np.uint32), c.astype(np.uint32))
+        ref = np.pad(ref, ((0, 0), (0, width - ref.shape[1])))
+        _check(got[rows], o.bf16_bits_to_f32(o.f32_to_bf16_bits_np(ref)), np.zeros(len(c), np.uint32), c.astype(np.uint32), width, fill)
+    # the rest in float32 on the GPU: same bf16 logits up to one rounding and the order of the sums
+    kv_t, q_t, w_t = torch.from_numpy(kvd).cuda(), torch.from_numpy(qd).cuda(), wb.float().cuda()
+    for r in range(nreq):
+        for t in range(first[r], first[r] + ntok[r]):
+            if ctx[t]:
+                ref = (torch.relu(q_t[t] @ kv_t[torch.from_numpy(perm[r].astype(np.int64)).cuda()].reshape(-1, D)[:ctx[t]].T) * w_t[t][:, None]).sum(0)
+                err = (logits[t, :ctx[t]].float() - ref).abs().max() / ref.pow(2).mean().sqrt().clamp_min(1e-6)
+                assert err.item() <= 0.05
