@@ -444,23 +444,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     }
                     if (MNM) {
                         // An MN-major operand is a [K, MN] buffer: a box is one swizzle atom (128 bytes of MN)
-                        // wide and BLOCK_K rows deep, neighbouring atoms along MN lie box_bytes apart.
-                        const uint32_t bar = smem_u32(&bars->full[stage]);
-                        mbar_arrive_expect_tx(bar, p.tx_ab);
-                        const int32_t ky = (int32_t)((GTYPE == kBatched ? t.batch * p.k_elems : 0u) + (uint32_t)kx);
+                        // wide and BLOCK_K rows deep, neighbouring atoms along MN lie box_bytes apart.  On a CTA pair
+                        // every CTA loads its own rows of A and its own half of B, as with K-major tiles.
+                        if (leader) mbar_arrive_expect_tx(smem_u32(&bars->full[stage]), CL * p.tx_ab);
+                        const uint32_t bar = CL == 1 ? smem_u32(&bars->full[stage]) : mapa(smem_u32(&bars->full[stage]), 0);
+                        auto load = [&](const CUtensorMap* tm, uint32_t dst, uint32_t x, uint32_t y) {
+                            if (CL == 1) tma_load_2d(tm, bar, dst, (int32_t)x, (int32_t)y);
+                            else tma_load_2d_pair(tm, bar, dst, (int32_t)x, (int32_t)y);
+                        };
+                        const uint32_t ky = (GTYPE == kBatched ? t.batch * p.k_elems : 0u) + (uint32_t)kx;
                         if (p.a_mn) {
                             const uint32_t mn0 = GTYPE == kBatched ? t.mn_a : t.a_row;
-                            for (uint32_t i = 0; i < p.a_boxes; ++i)
-                                tma_load_2d(&tm_a, bar, sa + i * p.box_bytes, (int32_t)(mn0 + i * p.box_elems), ky);
+                            for (uint32_t i = 0; i < p.a_boxes; ++i) load(&tm_a, sa + i * p.box_bytes, mn0 + i * p.box_elems, ky);
                         } else {
-                            tma_load_2d(&tm_a, bar, sa, kx, (int32_t)t.a_row);
+                            load(&tm_a, sa, (uint32_t)kx, t.a_row);
                         }
                         if (p.b_mn) {
-                            const uint32_t mn0 = GTYPE == kBatched ? t.n0 + p.b_row_offset : t.b_row;
-                            for (uint32_t i = 0; i < p.b_boxes; ++i)
-                                tma_load_2d(&tm_b, bar, sa + p.off_b + i * p.box_bytes, (int32_t)(mn0 + i * p.box_elems), ky);
+                            const uint32_t mn0 = (GTYPE == kBatched ? t.n0 + p.b_row_offset : t.b_row) + rank * b_rows_per_cta;
+                            for (uint32_t i = 0; i < p.b_boxes; ++i) load(&tm_b, sa + p.off_b + i * p.box_bytes, mn0 + i * p.box_elems, ky);
                         } else {
-                            tma_load_2d(&tm_b, bar, sa + p.off_b, kx, (int32_t)t.b_row);
+                            load(&tm_b, sa + p.off_b, (uint32_t)kx, t.b_row + rank * b_rows_per_cta);
                         }
                     } else if (CL == 1) {
                         const uint32_t bar = smem_u32(&bars->full[stage]);
@@ -1116,7 +1119,9 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     const uint32_t forced_cl = env_u32("DG_CLUSTER", 0);
     if (forced_cl == 1 || forced_cl == 2) cl = forced_cl;
     if (gtype == kContiguous && m / kBlockM > kMaxPairedBlocks) cl = 1;   // the in-kernel tile list is bounded
-    if (a_mn || b_mn) cl = 1;   // MN-major tiles are loaded atom by atom by one CTA
+    // MN-major tiles: BF16 GEMMs run on pairs as well (every CTA loads whole swizzle atoms of its share); FP8 atoms are
+    // 128 columns, and two of them per CTA would be wider than the accumulators beside the scale factors.
+    if ((a_mn || b_mn) && (kind != kBf16 || gtype != kNormal)) cl = 1;
     uint32_t dense_bn = 0;
     if (kind == kFp8 && (gtype == kNormal || gtype == kMasked) && gran_a == 128 && gran_b == 128 && !a_mn && !b_mn &&
         (gtype == kMasked || m > kBlockM) && forced_cl == 0 && env_u32("DG_BLOCK_N", 0) == 0)
@@ -1133,7 +1138,7 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     else if (gtype == kBatched) m_tiles_total = num_groups * ceil_div(m, tile_m);
     else m_tiles_total = ceil_div(m, tile_m);
     // an MN-major B is loaded in whole swizzle atoms of 128 bytes along N: 128 columns of FP8, 64 of BF16
-    p.block_n = dense_bn ? dense_bn : pick_block_n(kind, m_tiles_total, n, units, b_mn ? (kind == kBf16 ? 64u : 128u) : 32u);
+    p.block_n = dense_bn ? dense_bn : pick_block_n(kind, m_tiles_total, n, units, b_mn ? (kind == kBf16 ? 64u * cl : 128u) : 32u);
     p.num_m_blocks = ceil_div(m, tile_m);
     p.num_n_blocks = ceil_div(n, p.block_n);
     // Split-K for weight-streaming shapes (a single row block, long K): with one tile per SM at
@@ -1193,7 +1198,7 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     p.box_elems = kind == kBf16 ? 64u : 128u;
     p.box_bytes = 128u * block_k_rows;
     p.a_boxes = kBlockM / p.box_elems;
-    p.b_boxes = ceil_div(p.block_n, p.box_elems);
+    p.b_boxes = ceil_div(p.block_n / cl, p.box_elems);
     p.mn_kstep = (kind == kBf16 ? 16u : 32u) * 128u / 16u;
     p.k_elems = k;
     const uint32_t a_bytes = kBlockM * 128u, b_bytes = b_mn ? p.b_boxes * p.box_bytes : p.block_n / cl * 128u;
@@ -1535,6 +1540,7 @@ static int32_t run_gemm(const dg_operand_t* a, const dg_operand_t* b, dg_output_
     if (a_mn || b_mn) {
         if (kind == kFp8 && gtype == kNormal) return launch<kFp8, kNormal, 1, false, false, true>(plan, ta, tb, tsa, tsb, s);
         if (kind == kFp8 && gtype == kBatched) return launch<kFp8, kBatched, 1, false, false, true>(plan, ta, tb, tsa, tsb, s);
+        if (kind == kBf16 && gtype == kNormal && plan.cluster == 2) return launch<kBf16, kNormal, 2, false, false, true>(plan, ta, tb, tsa, tsb, s);
         if (kind == kBf16 && gtype == kNormal) return launch<kBf16, kNormal, 1, false, false, true>(plan, ta, tb, tsa, tsb, s);
         if (kind == kBf16 && gtype == kBatched) return launch<kBf16, kBatched, 1, false, false, true>(plan, ta, tb, tsa, tsb, s);
     }

@@ -198,3 +198,23 @@ def test_contiguous_gemm_recorded_into_a_cuda_graph():
             assert not got[rows].any()
         else:
             assert_close_to_oracle(got[rows], bf16_round(o.gemm_ref(ga, gw, rows=rows, n=n, b_row0=e * n)), "fp8", f"block {blk}")
+
+
+@pytest.mark.parametrize("layout", ["nn", "tn", "tt"])
+@pytest.mark.parametrize("m,n,k,f32", [(129, 64, 64, False), (257, 1048, 320, False), (640, 264, 2048, True), (512, 2048, 192, True)])
+def test_bf16_mn_major_views_on_cta_pairs(layout, m, n, k, f32):
+    """BF16 with more than one 128-row block runs on CTA pairs: second CTAs without rows or columns, a second half of B
+    outside the tensor, and accumulation into f32."""
+    from helpers import bf16_operand
+    a, fa = bf16_operand(randn((m, k), m))
+    b, fb = bf16_operand(randn((n, k), n + 1))
+    out = new_output(m, n, f32=f32, fill=1.5 if f32 else None)
+    if layout == "nn":
+        gemm_nn(a, mn_view(b), out, accumulate=f32)
+    elif layout == "tn":
+        gemm_tn(mn_view(a), b, out, accumulate=f32)
+    else:
+        gemm_tt(mn_view(a), mn_view(b), out, accumulate=f32)
+    poll_device_status()
+    ref = o.gemm_f32_ref(fa, fb)
+    assert_close_to_oracle(to_f32(out), ref + 1.5 if f32 else bf16_round(ref), "bf16", f"{layout} {m}x{n}x{k}")
