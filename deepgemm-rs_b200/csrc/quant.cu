@@ -34,7 +34,7 @@ template <uint32_t R, uint32_t G, bool FP4, bool SWIGLU = false, bool STOCH = fa
 __global__ void __launch_bounds__(256) quant_mx_kernel(const float* __restrict__ x, uint32_t m, uint32_t k,
                                                       uint8_t* __restrict__ data, uint32_t* __restrict__ sf,
                                                       uint32_t sf_cols, uint32_t num_spans, uint32_t num_row_blocks,
-                                                      uint64_t src_pitch, uint32_t seed) {
+                                                      uint64_t src_pitch, uint32_t seed, const int32_t* __restrict__ block_expert) {
     constexpr uint32_t kLoads = G / 32;                   // float4 loads per lane per row
     // Row pitch of a plain f32 input: K itself unless PITCHED (quantize_output_fp8), as a 32-bit value so that the
     // row offset is one widening multiply.  A run-time 64-bit select in its place made the per-128 kernel 35 %
@@ -53,6 +53,8 @@ __global__ void __launch_bounds__(256) quant_mx_kernel(const float* __restrict__
     // 8 * 4G contiguous floats of each row.
     const uint32_t span = warp_global % num_spans;
     const uint32_t row0 = (warp_global / num_spans) * R;
+    // rows of a 128-row block that no expert owns: nobody reads their codes
+    if (SWIGLU && block_expert && __ldg(block_expert + row0 / 128u) < 0) return;
     const uint32_t num_groups = k / G;
     const uint32_t groups_here = min(4u, num_groups - span * 4u);
     const uint32_t col0 = span * 4u * G;
@@ -252,7 +254,7 @@ static bool eight_rows_per_warp(uint32_t m, uint32_t k) {
 // for its predecessor itself and lets its successor set up early).
 template <uint32_t R, uint32_t G, bool FP4, bool SWIGLU, bool STOCH, bool PITCHED>
 static int32_t launch_quant_rows(const void* x, uint32_t m, uint32_t k, void* data_out, uint32_t* sf_out, uint64_t src_pitch,
-                                 uint32_t seed, cudaStream_t s) {
+                                 uint32_t seed, cudaStream_t s, const int32_t* block_expert = nullptr) {
     const uint32_t sf_cols = align_up(m, 4);
     const uint32_t num_spans = ceil_div(k / G, 4);
     const uint32_t num_row_blocks = ceil_div(sf_cols, R);
@@ -267,20 +269,20 @@ static int32_t launch_quant_rows(const void* x, uint32_t m, uint32_t k, void* da
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     DG_CUDA_CHECK(cudaLaunchKernelEx(&cfg, quant_mx_kernel<R, G, FP4, SWIGLU, STOCH, PITCHED>, static_cast<const float*>(x), m, k,
-                                     static_cast<uint8_t*>(data_out), sf_out, sf_cols, num_spans, num_row_blocks, src_pitch, seed));
+                                     static_cast<uint8_t*>(data_out), sf_out, sf_cols, num_spans, num_row_blocks, src_pitch, seed, block_expert));
     note_launch();
     return DG_OK;
 }
 
 template <uint32_t G, bool FP4, bool SWIGLU = false, bool STOCH = false, bool PITCHED = false>
 static int32_t launch_quant_kernel(const void* x, uint32_t m, uint32_t k, void* data_out, uint32_t* sf_out, uint64_t src_pitch,
-                                   uint32_t seed, cudaStream_t s) {
+                                   uint32_t seed, cudaStream_t s, const int32_t* block_expert = nullptr) {
     // SwiGLU forms its values from twice the loads: 2 rows are best at every size (24320 x 2048: 94 / 66 / 62 us)
     if constexpr (!SWIGLU && !STOCH && !PITCHED && (FP4 || G == 128)) {
         if (eight_rows_per_warp<G, FP4>(m, k))
-            return launch_quant_rows<8, G, FP4, SWIGLU, STOCH, PITCHED>(x, m, k, data_out, sf_out, src_pitch, seed, s);
+            return launch_quant_rows<8, G, FP4, SWIGLU, STOCH, PITCHED>(x, m, k, data_out, sf_out, src_pitch, seed, s, block_expert);
     }
-    return launch_quant_rows<2, G, FP4, SWIGLU, STOCH, PITCHED>(x, m, k, data_out, sf_out, src_pitch, seed, s);
+    return launch_quant_rows<2, G, FP4, SWIGLU, STOCH, PITCHED>(x, m, k, data_out, sf_out, src_pitch, seed, s, block_expert);
 }
 
 static int32_t launch_quant(const float* x, uint32_t m, uint32_t k, int32_t dtype, uint32_t gran, void* data_out,
@@ -294,20 +296,26 @@ static int32_t launch_quant(const float* x, uint32_t m, uint32_t k, int32_t dtyp
 
 extern "C" {
 
-int32_t dg_swiglu_quant(const void* gate_up_bf16, uint64_t pitch, uint32_t m, uint32_t inter, uint32_t gran, void* data_out,
-                        uint32_t* sf_out, void* stream) {
+int32_t dg_swiglu_quant_grouped(const void* gate_up_bf16, uint64_t pitch, uint32_t m, uint32_t inter, uint32_t gran,
+                                const int32_t* block_expert, void* data_out, uint32_t* sf_out, void* stream) {
     if (!gate_up_bf16 || !data_out || !sf_out) return dg::fail(DG_ERR_INVALID_ARG, "swiglu_quant: null buffer");
     if (gran != 32 && gran != 128) return dg::fail(DG_ERR_INVALID_ARG, "swiglu_quant: SF granularity must be 32 or 128");
     if (m == 0 || inter == 0 || inter % gran != 0 || inter % 4 != 0)
         return dg::fail(DG_ERR_INVALID_ARG, "swiglu_quant: the intermediate width (%u) must be a positive multiple of the granularity", inter);
     if (pitch < 2ull * inter || pitch % 4 != 0 || (reinterpret_cast<uintptr_t>(gate_up_bf16) & 7u))
         return dg::fail(DG_ERR_INVALID_ARG, "swiglu_quant: the row pitch must cover 2 x %u columns and keep rows 8-byte aligned", inter);
+    if (block_expert && m % 128 != 0) return dg::fail(DG_ERR_INVALID_ARG, "swiglu_quant: grouped rows (%u) come in blocks of 128", m);
     const dg::DeviceInfo* dev;
     int32_t st = dg::current_device(&dev);
     if (st != DG_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    return gran == 32 ? dg::launch_quant_kernel<32, false, true>(gate_up_bf16, m, inter, data_out, sf_out, pitch, 0, s)
-                      : dg::launch_quant_kernel<128, false, true>(gate_up_bf16, m, inter, data_out, sf_out, pitch, 0, s);
+    return gran == 32 ? dg::launch_quant_kernel<32, false, true>(gate_up_bf16, m, inter, data_out, sf_out, pitch, 0, s, block_expert)
+                      : dg::launch_quant_kernel<128, false, true>(gate_up_bf16, m, inter, data_out, sf_out, pitch, 0, s, block_expert);
+}
+
+int32_t dg_swiglu_quant(const void* gate_up_bf16, uint64_t pitch, uint32_t m, uint32_t inter, uint32_t gran, void* data_out,
+                        uint32_t* sf_out, void* stream) {
+    return dg_swiglu_quant_grouped(gate_up_bf16, pitch, m, inter, gran, nullptr, data_out, sf_out, stream);
 }
 
 int32_t dg_quant_mx(const float* x, uint32_t m, uint32_t k, int32_t dtype, uint32_t gran, void* data_out,

@@ -87,6 +87,7 @@ def load(build_if_missing=True):
     L.dg_quant_mx_host.argtypes = [vp, u32, u32, i32, u32, vp, vp, vp]
     L.dg_quant_mx_host_static.argtypes = [vp, u32, u32, i32, u32, vp, vp, vp]
     L.dg_swiglu_quant.argtypes = [vp, u64, u32, u32, u32, vp, vp, vp]
+    L.dg_swiglu_quant_grouped.argtypes = [vp, u64, u32, u32, u32, vp, vp, vp, vp]
     L.dg_dequant_mx.argtypes = [vp, C.POINTER(SfTensorC), u32, u32, i32, vp, vp]
     L.dg_transform_sf.argtypes = [vp, u32, u32, vp, vp]
     L.dg_transform_sf_host.argtypes = [vp, u32, u32, vp, vp]
@@ -97,6 +98,7 @@ def load(build_if_missing=True):
     L.dg_mqa_logits_paged.argtypes = [opp, vp, vp, vp, u32, u32, vp, vp, vp, u32, u32, u32, u32, vp, u32, vp]
     L.dg_gather_rows.argtypes = [vp, u64, vp, vp, u64, u32, u32, vp]
     L.dg_gather_sf.argtypes = [vp, u64, u64, vp, vp, u64, u64, u32, u32, vp]
+    L.dg_moe_gather.argtypes = [vp, u64, u32, vp, u32, u64, vp, vp, u32, u32, vp, vp, vp]
     L.dg_moe_plan.argtypes = [vp, u32, u32, u32, u32, u32, vp, vp, vp, vp, vp, vp, vp]
     L.dg_moe_combine.argtypes = [vp, u64, vp, vp, vp, u64, u32, u32, u32, vp]
     L.dg_peer_alloc.argtypes = [u64, C.POINTER(vp)]

@@ -25,7 +25,7 @@ import torch.distributed as dist
 
 from . import _lib
 from .api import (_check, _stream_ptr, m_grouped_gemm_nt_contiguous, m_grouped_gemm_nt_contiguous_gather,
-                  m_grouped_gemm_nt_contiguous_rowptr, m_grouped_gemm_nt_contiguous_scatter, swiglu_quant)
+                  m_grouped_gemm_nt_contiguous_rowptr, m_grouped_gemm_nt_contiguous_scatter, sf_shape)
 from .types import Dtype, Operand, Output, SfGran, SfTensor
 
 BLOCK = 128  # rows per m_indices entry (heuristics::mk_alignment_for_contiguous_layout)
@@ -192,6 +192,16 @@ def sf_permute(sf, idx):
     return SfTensor(sf.rows, idx.numel(), sf.gran, buf)
 
 
+def _gather_tokens(x, x_sf, plan):
+    """Token rows and scale-factor columns of a padded layout in one pass (blocks without an owner stay unwritten)."""
+    rows = torch.empty((plan.capacity, x.shape[1]), dtype=x.dtype, device=x.device)
+    buf = torch.empty((x_sf.rows, plan.capacity), dtype=torch.int32, device=x.device)
+    _check(_lib.load().dg_moe_gather(x.data_ptr(), x.stride(0) * x.element_size(), x.shape[1] * x.element_size(), x_sf.buf.data_ptr(),
+                                     x_sf.rows, x_sf.cols, plan.slot_src.data_ptr(), plan.block_expert.data_ptr(), BLOCK, plan.capacity,
+                                     rows.data_ptr(), buf.data_ptr(), _stream_ptr(None)))
+    return rows, SfTensor(x_sf.rows, plan.capacity, x_sf.gran, buf)
+
+
 def combine(src, pos, weights, out=None):
     """out[t] = sum_j weights[t, j] * src[pos[t, j]] (bf16 rows, f32 accumulation)."""
     tokens, topk = pos.shape
@@ -222,15 +232,17 @@ class GroupedMoEFfn:
         tokens, topk = topk_idx.shape
         hidden, out_dim = x.shape[1], self.w2.rows
         p = device_plan(topk_idx, self.num_experts, BLOCK, div=topk)
-        a = gather_rows(x, p.slot_src)
-        a_sf = sf_permute(x_sf, p.slot_src)
+        a, a_sf = _gather_tokens(x, x_sf, p)
         gate_up = torch.empty((p.capacity, 2 * self.inter), dtype=torch.bfloat16, device=x.device)
         m_grouped_gemm_nt_contiguous(Operand.k_major(self.w13.dtype, p.capacity, hidden, hidden, a_sf, a), self.w13,
                                      Output(Dtype.Bf16, p.capacity, 2 * self.inter, 2 * self.inter, gate_up), p.block_expert,
                                      self.num_experts)
-        # rows of unused blocks hold whatever the allocation held: they are quantised like the others
-        # and never read, because the second GEMM skips their blocks and the combine step their slots
-        h, h_sf = swiglu_quant(gate_up, p.capacity, self.inter, self.gran)
+        # blocks that no expert owns are skipped here like in both GEMMs; the combine step reads none of their slots
+        h = torch.empty((p.capacity, self.inter), dtype=torch.uint8, device=x.device)
+        rows, cols = sf_shape(p.capacity, self.inter, self.gran)
+        h_sf = SfTensor(rows, cols, SfGran(int(self.gran)), torch.empty((rows, cols), dtype=torch.int32, device=x.device))
+        _check(_lib.load().dg_swiglu_quant_grouped(gate_up.data_ptr(), gate_up.stride(0), p.capacity, self.inter, int(self.gran),
+                                                   p.block_expert.data_ptr(), h.data_ptr(), h_sf.buf.data_ptr(), _stream_ptr(None)))
         d = torch.empty((p.capacity, out_dim), dtype=torch.bfloat16, device=x.device)
         m_grouped_gemm_nt_contiguous(Operand.k_major(Dtype.Fp8, p.capacity, self.inter, self.inter, h_sf, h), self.w2,
                                      Output(Dtype.Bf16, p.capacity, out_dim, out_dim, d), p.block_expert, self.num_experts)
@@ -319,15 +331,15 @@ class ExpertParallelMoE:
         if self.world == 1 and not (self.single_rank_transport and self.transport == "push"):
             # one device-side plan straight into the padded layout; no host synchronisation
             p = device_plan(topk_idx, self.num_experts, BLOCK, div=topk)
-            a_sf = sf_permute(x_sf, p.slot_src)
             d = torch.empty((p.capacity, n_out), dtype=torch.bfloat16, device=x.device)
             if self.w.dtype == Dtype.Fp8 and x.stride(0) == k and _gather_in_gemm():
                 # the GEMM's producer fetches the token rows itself (four per TMA instruction): no permuted copy
+                a_sf = sf_permute(x_sf, p.slot_src)
                 a_op = Operand.k_major(self.w.dtype, p.capacity, k_elems, k_elems, a_sf, x)
                 m_grouped_gemm_nt_contiguous_gather(a_op, p.slot_src, tokens, self.w, Output(Dtype.Bf16, p.capacity, n_out, n_out, d),
                                                     p.block_expert, self.e_local)
             else:
-                a = gather_rows(x, p.slot_src)
+                a, a_sf = _gather_tokens(x, x_sf, p)
                 a_op = Operand.k_major(self.w.dtype, p.capacity, k_elems, k_elems, a_sf, a)
                 m_grouped_gemm_nt_contiguous(a_op, self.w, Output(Dtype.Bf16, p.capacity, n_out, n_out, d), p.block_expert,
                                              self.e_local)

@@ -127,6 +127,8 @@ extern "C" {
                                   sf_out: *mut u32, stream: Stream) -> i32;
     pub fn dg_swiglu_quant(gate_up_bf16: *const c_void, pitch: u64, m: u32, inter: u32, gran: u32, data_out: *mut c_void,
                            sf_out: *mut u32, stream: Stream) -> i32;
+    pub fn dg_swiglu_quant_grouped(gate_up_bf16: *const c_void, pitch: u64, m: u32, inter: u32, gran: u32, block_expert: *const i32,
+                                   data_out: *mut c_void, sf_out: *mut u32, stream: Stream) -> i32;
 
     // ---- MQA logits (api.rs:1614-1941; fp32 contract api_sm90_mqa.rs:5-31)
     pub fn dg_mqa_logits_f32(q: *const c_void, kv: *const c_void, kv_scale: *const f32, weights: *const f32, cu_k_start: *const u32,
@@ -145,6 +147,9 @@ extern "C" {
                           n_rows: u32, row_bytes: u32, stream: Stream) -> i32;
     pub fn dg_gather_sf(src: *const u32, src_row_stride: u64, src_col_stride: u64, idx: *const i32, dst: *mut u32,
                         dst_row_stride: u64, dst_col_stride: u64, sf_rows: u32, n: u32, stream: Stream) -> i32;
+    pub fn dg_moe_gather(x: *const c_void, x_pitch_bytes: u64, row_bytes: u32, x_sf: *const u32, sf_rows: u32, sf_cols: u64,
+                         slot_src: *const i32, block_expert: *const i32, align: u32, capacity: u32, rows_out: *mut c_void,
+                         sf_out: *mut u32, stream: Stream) -> i32;
     pub fn dg_moe_plan(expert_of_row: *const i32, n_rows: u32, num_experts: u32, align: u32, div: u32, capacity: u32,
                        counts: *mut i32, offsets: *mut i32, cursors: *mut i32, slot_src: *mut i32, slot_of_row: *mut i32,
                        block_expert: *mut i32, stream: Stream) -> i32;

@@ -283,6 +283,12 @@ DG_API int32_t dg_gather_rows(const void* src, uint64_t src_pitch_bytes, const i
 DG_API int32_t dg_gather_sf(const uint32_t* src, uint64_t src_row_stride, uint64_t src_col_stride, const int32_t* idx,
                             uint32_t* dst, uint64_t dst_row_stride, uint64_t dst_col_stride, uint32_t sf_rows, uint32_t n,
                             void* stream);
+/* Both of them for a whole padded layout (dg_moe_plan's slot_src and block_expert for blocks of `align` slots, a multiple
+ * of 32) in one pass: rows_out [capacity, row_bytes] and sf_out [sf_rows, capacity]; slots of blocks that no expert owns
+ * are not written. */
+DG_API int32_t dg_moe_gather(const void* x, uint64_t x_pitch_bytes, uint32_t row_bytes, const uint32_t* x_sf, uint32_t sf_rows,
+                             uint64_t sf_cols, const int32_t* slot_src, const int32_t* block_expert, uint32_t align,
+                             uint32_t capacity, void* rows_out, uint32_t* sf_out, void* stream);
 /* Grouping plan on the device (no host synchronisation): rows with expert ids expert_of_row[r]
  * (negative = drop) are assigned slots so that each expert's rows are contiguous and every group
  * is padded to `align` rows (128 for the grouped GEMM, 1 for a plain sort by expert).
@@ -308,6 +314,10 @@ DG_API int32_t dg_moe_combine(const void* src_bf16, uint64_t src_pitch, const in
  * Arithmetic as in the golden model's fused path (golden.rs:569-577): f32 on the bf16 values, no clamp. */
 DG_API int32_t dg_swiglu_quant(const void* gate_up_bf16, uint64_t pitch, uint32_t m, uint32_t inter, uint32_t gran,
                                void* data_out, uint32_t* sf_out, void* stream);
+/* The same for a padded contiguous MoE layout: block_expert (int32, one entry per 128 rows, m a multiple of 128)
+ * names the owner of every block; rows of blocks with a negative entry are neither read nor written. */
+DG_API int32_t dg_swiglu_quant_grouped(const void* gate_up_bf16, uint64_t pitch, uint32_t m, uint32_t inter, uint32_t gran,
+                                       const int32_t* block_expert, void* data_out, uint32_t* sf_out, void* stream);
 
 /* ---- expert parallelism over peer memory (extensions; the reference runs on one GPU and has no
  * counterpart for any entry of this block) ---------------------------------------------------

@@ -77,3 +77,20 @@ def test_moe_ffn_layer_matches_oracle():
     assert o.calc_diff(got, want) <= 1e-3
     rms = np.sqrt((want.astype(np.float64) ** 2).mean())
     assert np.abs(got - want).max() <= 0.05 * rms
+
+
+@pytest.mark.parametrize("owners", [[0, -1, 2, -1], [-1, -1], [3]])
+def test_swiglu_quant_grouped_skips_unowned_blocks(owners):
+    from deepgemm import _lib
+    m, inter = 128 * len(owners), 384
+    gate_up = torch.from_numpy(randn((m, 2 * inter), 4)).to(torch.bfloat16).cuda()
+    want, want_sf = swiglu_quant(gate_up, m, inter, 128)
+    data = torch.full((m, inter), 0xEE, dtype=torch.uint8, device="cuda")
+    sf = torch.full((want_sf.rows, want_sf.cols), -7, dtype=torch.int32, device="cuda")
+    be = torch.tensor(owners, dtype=torch.int32, device="cuda")
+    st = _lib.load().dg_swiglu_quant_grouped(gate_up.data_ptr(), gate_up.stride(0), m, inter, 128, be.data_ptr(), data.data_ptr(),
+                                             sf.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    owned = (be >= 0).repeat_interleave(128)
+    assert torch.equal(data[owned], want[owned]) and (data[~owned] == 0xEE).all()
+    assert torch.equal(sf[:, owned], want_sf.buf[:, owned]) and (sf[:, ~owned] == -7).all()
