@@ -28,6 +28,7 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <unistd.h>
 
 namespace dg {
 
@@ -1049,8 +1050,16 @@ static uint32_t* tile_counters(const DeviceInfo* dev) {
     return dev->tile_pool + 2u * (next[dev->device & 63]++ % kTilePoolPairs);
 }
 
+// A GEMM consults some twenty DG_* variables, which are hardly ever set: one pass over the environment per call says
+// whether any is, and only then are they looked up.
+static thread_local bool t_any_dg_env = true;
+static void note_env() {
+    t_any_dg_env = false;
+    for (char** e = environ; e && *e; ++e)
+        if ((*e)[0] == 'D' && (*e)[1] == 'G' && (*e)[2] == '_') { t_any_dg_env = true; return; }
+}
 static uint32_t env_u32(const char* name, uint32_t dflt) {
-    const char* v = getenv(name);
+    const char* v = t_any_dg_env ? getenv(name) : nullptr;
     return v && *v ? (uint32_t)strtoul(v, nullptr, 10) : dflt;
 }
 
@@ -1099,6 +1108,7 @@ static void pick_dense_fp8_tile(uint32_t m, uint32_t groups, uint32_t n, uint32_
 static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k, uint32_t num_groups,
                          uint32_t expected_m, uint32_t gran_a, uint32_t gran_b, const DeviceInfo* dev, Plan* plan,
                          bool allow_dynamic = true, bool a_mn = false, bool b_mn = false) {
+    note_env();
     GemmParams& p = plan->p;
     p = GemmParams{};
     const uint32_t sms = (uint32_t)dev->sm_count;
