@@ -408,6 +408,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     const uint32_t n_runs = kPairedContig ? *reinterpret_cast<volatile uint32_t*>(&bars->n_runs) : 0u;
 
     auto stage_addr = [&](uint32_t s) { return stages_base + s * p.stage_bytes; };
+    // SF rows of a k-block: chunks of 128 words (512 bytes), A's first and B's right behind them.
+    constexpr uint32_t kSfSub = KIND == kFp4 ? 2u : 1u;      // SF rows per k-block (p.sf_sub)
+    // One thread: the chunks of the stage at `sa` into the SF set's columns.  Straight-line, the descriptors stepping by
+    // a chunk: as loops over run-time counts the copies of a k-block cost the issuing thread some 350 cycles, three or six alike.
+    auto copy_sf = [&](uint32_t sa, uint32_t set) {
+        const uint32_t col = tmem + sf_set_col(set);
+        const uint64_t d = make_sf_desc(sa + p.off_sfa);
+#pragma unroll
+        for (uint32_t c = 0; c < kSfSub; ++c) tc_cp_32x128b_warpx4<CL>(col + kSfaOff + c * 4u, d + c * 32u);
+#pragma unroll
+        for (uint32_t c = 0; c < kSfSub; ++c) tc_cp_32x128b_warpx4<CL>(col + kSfbOff + c * 4u, d + (kSfSub + c) * 32u);
+        if (p.sfb_chunks > 1u) {
+#pragma unroll
+            for (uint32_t c = kSfSub; c < 2u * kSfSub; ++c) tc_cp_32x128b_warpx4<CL>(col + kSfbOff + c * 4u, d + (kSfSub + c) * 32u);
+        }
+    };
 
     if (warp == 0) {
         // ===================================================== TMA producer (warp-converged, one lane issues)
@@ -523,9 +539,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 if (kConsLane || elect_one()) {
                     if (kHasSf && !SFW && (kb & p.sf_load_mask) == 0) {
                         // in order with the MMAs in the tensor pipe: the copy may overwrite the set the MMAs before it read
-                        const uint32_t na = p.sf_sub, nb = p.sf_sub * p.sfb_chunks;
-                        for (uint32_t c = 0; c < na; ++c) tc_cp_32x128b_warpx4<CL>(sfa_col + c * 4u, make_sf_desc(sa + p.off_sfa + c * 512u));
-                        for (uint32_t c = 0; c < nb; ++c) tc_cp_32x128b_warpx4<CL>(sfb_col + c * 4u, make_sf_desc(sa + p.off_sfb + c * 512u));
+                        copy_sf(sa, sf_set);
                     }
                     // K-major tile: 8-row groups 1024 B apart.  MN-major tile: 8 K rows of an atom are 1024 B
                     // apart (SBO), atoms along MN box_bytes apart (LBO).
@@ -602,27 +616,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     ok = DG_WARP_WAIT(smem_u32(&bars->sf_full[stage]), parity, wc, kWaitFull);
                     if (!ok) break;
                     const uint32_t sa = stage_addr(stage);
-                    uint32_t* sfa = reinterpret_cast<uint32_t*>(smem_raw + (sa + p.off_sfa - smem_u32(smem_raw)));
-                    uint32_t* sfb = reinterpret_cast<uint32_t*>(smem_raw + (sa + p.off_sfb - smem_u32(smem_raw)));
-                    const uint32_t na = p.sf_sub, nb = p.sf_sub * p.sfb_chunks;
-                    // Up to 6 chunks of 128 words: word of row 32*i + lane -> position lane*4 + i.
+                    uint32_t* sf = reinterpret_cast<uint32_t*>(smem_raw + (sa + p.off_sfa - smem_u32(smem_raw)));
+                    // Every chunk of 128 words: word of row 32*i + lane -> position lane*4 + i.
                     // All loads are issued before the first store.
-                    uint4 v[6];
+                    constexpr uint32_t kChunks = 3u * kSfSub;          // one of A and up to two of B per SF row
+                    uint4 v[kChunks];
 #pragma unroll
-                    for (uint32_t c = 0; c < 6; ++c) {
-                        if (c < na + nb) {
-                            const uint32_t* q = c < na ? sfa + c * 128u : sfb + (c - na) * 128u;
-                            v[c] = make_uint4(q[lane], q[32 + lane], q[64 + lane], q[96 + lane]);
-                        }
-                    }
+                    for (uint32_t c = 0; c < kChunks; ++c)
+                        if (c < 2u * kSfSub || p.sfb_chunks > 1u)
+                            v[c] = make_uint4(sf[c * 128u + lane], sf[c * 128u + 32u + lane], sf[c * 128u + 64u + lane], sf[c * 128u + 96u + lane]);
                     __syncwarp();
 #pragma unroll
-                    for (uint32_t c = 0; c < 6; ++c) {
-                        if (c < na + nb) {
-                            uint32_t* q = c < na ? sfa + c * 128u : sfb + (c - na) * 128u;
-                            *reinterpret_cast<uint4*>(q + lane * 4u) = v[c];
-                        }
-                    }
+                    for (uint32_t c = 0; c < kChunks; ++c)
+                        if (c < 2u * kSfSub || p.sfb_chunks > 1u) *reinterpret_cast<uint4*>(sf + c * 128u + lane * 4u) = v[c];
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (!SFW) {
@@ -635,9 +641,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                         if (n_sf >= 2u && !(ok = DG_WARP_WAIT(smem_u32(&bars->sf_free[set]), ((n_sf >> 1) - 1u) & 1u, wc, kWaitSfFree))) break;
                         tc_fence_after();
                         if (elect_one()) {
-                            const uint32_t sfa_col = tmem + sf_set_col(set) + kSfaOff, sfb_col = tmem + sf_set_col(set) + kSfbOff;
-                            for (uint32_t c = 0; c < na; ++c) tc_cp_32x128b_warpx4<CL>(sfa_col + c * 4u, make_sf_desc(sa + p.off_sfa + c * 512u));
-                            for (uint32_t c = 0; c < nb; ++c) tc_cp_32x128b_warpx4<CL>(sfb_col + c * 4u, make_sf_desc(sa + p.off_sfb + c * 512u));
+                            copy_sf(sa, set);
                             tc_commit<CL>(smem_u32(&bars->sf_ready[stage]));
                         }
                         __syncwarp();

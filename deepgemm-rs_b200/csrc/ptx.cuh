@@ -83,8 +83,11 @@ __device__ __forceinline__ uint32_t mapa(uint32_t local_addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
     return r;
 }
+// The release is at the instruction's default scope: as .release.cluster this arrive held its warp for 1500 to 1640
+// cycles on B200 (the partner's scale-factor warp then set the pace of a CTA pair).  What it publishes is read in the
+// CTA that arrives -- its own shared memory, which its own tensor core reads behind a proxy fence, and its own TMEM.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 // ---------------------------------------------------------------- mbarrier
