@@ -38,6 +38,7 @@
 #include "host.h"
 #include "ptx.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 
 namespace dg {
@@ -919,15 +920,18 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
     p.ep_groups = dec ? 4u : three_groups ? 3u : block_q % 4 == 0 ? 4u : block_q % 2 == 0 ? 2u : 1u;
     p.unit = num_heads % 16 == 0 ? 16u : 4u;
     p.num_q_blocks = ceil_div(num_tokens, block_q);
-    // Contiguous kv: the work items are query blocks, each over its whole kv range.  With fewer query blocks than
-    // twice the SMs (a short prefill chunk, a handful of queries) the range is cut into pieces of at least eight
-    // kv blocks, so that every SM gets work.
+    // Contiguous kv: the work items are query blocks, each over its whole kv range or cut into pieces of at least eight kv
+    // blocks.  The number of pieces minimises the kv blocks of the busiest SM, two more counted per item for its
+    // query tile and weights.  (Pieces only below two items per SM, as before, left 334 query blocks, 2.26 per SM, at the
+    // pace of the SMs that had three.)
     p.kv_splits = 1;
-    if (!PAGED && p.num_q_blocks < 2u * (uint32_t)dev->sm_count) {
-        const uint32_t kv_blocks = ceil_div(num_kv, kMqaBlockKv);
-        const uint32_t want = ceil_div(2u * (uint32_t)dev->sm_count, p.num_q_blocks);
-        const uint32_t most = kv_blocks / 8u > 1u ? kv_blocks / 8u : 1u;
-        p.kv_splits = want < most ? want : most;
+    if (!PAGED) {
+        const uint32_t kv_blocks = ceil_div(num_kv, kMqaBlockKv), sms = (uint32_t)dev->sm_count;
+        uint64_t best = ~0ull;
+        for (uint32_t s = 1; s <= std::max(1u, kv_blocks / 8u) && (s == 1u || p.num_q_blocks * (s - 1u) < 8u * sms); ++s) {
+            const uint64_t cost = (uint64_t)ceil_div(p.num_q_blocks * s, sms) * (ceil_div(kv_blocks, s) + 2u);
+            if (cost < best) { best = cost; p.kv_splits = s; }
+        }
     }
     p.row_bytes = FP4 ? head_dim / 2 : head_dim;
     p.sbo = 8 * p.row_bytes;
