@@ -411,7 +411,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                                 tc_cp_32x128b_warpx4(tmem + kMqaSfbCol + c * 4u, make_sf_desc(qaddr + p.q_sf_off + c * 512u));
                         tc_cp_32x128b_warpx4(tmem + kMqaSfaCol, make_sf_desc(kaddr + p.kv_sf_off));
                     }
-                    for (uint32_t m = 0; m < p.num_mma; ++m) {
+                    auto mma = [&](uint32_t m) {
                         if (SCALED && FP4)      // 64 elements per MMA: half-word (m & 1) of the row's scale word
                             tc_mma_mxf4(d_tmem, kv_desc + 2u * m, q_desc + 2u * m, idesc_with_sf_ids(idesc, (m & 1u) * 2u, (m & 1u) * 2u),
                                         m != 0u, tmem + kMqaSfaCol, tmem + kMqaSfbCol);
@@ -420,7 +420,12 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                                         tmem + kMqaSfaCol, tmem + kMqaSfbCol);
                         else
                             tc_mma_f8(d_tmem, kv_desc + 2u * m, q_desc + 2u * m, idesc, m != 0u);
-                    }
+                    };
+                    // straight-line (one, two or four by the bytes of a row): as a loop over a run-time count the MMAs and
+                    // commits of a block took the issuer 690 cycles, and decode ran at the issuer's pace
+                    mma(0);
+                    if (p.num_mma > 1u) mma(1);
+                    if (p.num_mma > 2u) { mma(2); mma(3); }
                     tc_commit(smem_u32(&bars->kv_empty[stage]));
                     tc_commit(smem_u32(&bars->tmem_full[as]));
                     if (kb + 1 == k.kb1) tc_commit(smem_u32(&bars->q_empty[qs]));
