@@ -170,8 +170,7 @@ struct Scheduler {
         t.kb0 = 0; t.kb1 = p.num_k_blocks; t.split = 0;
         if (GTYPE == kContiguous && CL == 2) {
             // m-tiles come from the list built at kernel start: a pair of 128-row blocks of one
-            // expert, or a single block whose partner rows (the next block, another expert's) are
-            // computed by the second CTA and dropped.
+            // expert, or a single block whose second CTA works on rows of zeros that are dropped.
             // Tile order: one expert after the other; inside an expert its m-tiles are fastest, so
             // the tiles that share a weight tile run next to each other and the expert's few A
             // blocks are reused across all its n-blocks.
@@ -186,7 +185,9 @@ struct Scheduler {
             const uint32_t nb = rem / rows, mt = mt0 + (rem - nb * rows);
             const uint32_t entry = mtiles[mt], blk = entry & 0x7fffu;
             const bool paired = (entry & 0x8000u) != 0;
-            t.a_row = (blk + rank) * kBlockM;
+            // a block without a partner: the second CTA loads rows past the end, which the copies fill with zeros -- its
+            // products belong to nobody, and zeros cost the tensor cores and the memory system least
+            t.a_row = (rank == 0 || paired) ? (blk + rank) * kBlockM : p.m;
             t.row_end = (rank == 0 || paired) ? p.m : 0u;
             t.n0 = nb * p.block_n; t.tail = p.tail_n != 0u && nb + 1u == p.num_n_blocks;
             t.b_row = (uint32_t)__ldg(p.layout + blk) * p.b_group_rows + p.b_row_offset + t.n0;
@@ -295,12 +296,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     constexpr bool kHasSf = KIND != kBf16;
     static_assert(!(SFW && CL == 2), "the SF warp copies scale factors only on single CTAs");
     static_assert(!GA || (GTYPE == kContiguous && CL == 1 && !SPLIT && !MNM && KIND == kFp8), "gathered A rows: contiguous FP8, single CTAs");
-    // Whether one elected lane runs the MMA issuer's k-loop alone (no warp-wide vote and re-convergence per
-    // k-block).  Measured on one B200, warp-wide -> single lane: FP4 3470 -> 4200 TFLOPS, masked FP8 1009 -> 1052,
-    // split-K FP8 at M = 128 2 to 7 % faster, the contiguous grouped GEMM on 208-wide tiles (five stages) 1842 ->
-    // 1994 (on 224-wide tiles, four stages, where the pipeline depth bounds it, 1849 -> 1809); dense FP8 on CTA
-    // pairs 1950 -> 1925, so pairs keep the warp-wide loop.
-    constexpr bool kConsLane = KIND == kFp4 || SPLIT || GTYPE == kMasked || ((GTYPE == kNormal || GTYPE == kContiguous) && CL == 1);
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // Dynamic shared memory: [barriers (512 B, padded to 1024)] [stage 0] [stage 1] ...
     // (identical offsets in both CTAs of a pair: the launch gives every CTA the same window offset)
@@ -509,6 +504,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         uint32_t sf_set = 1;   // SF set the MMAs read; it changes at every SF k-block (the first one takes set 0)
         // The tile walk is done by the whole warp, the k-loop of a tile by one elected lane alone: warp-wide votes
         // and re-convergence on every k-block cost the issuer more than the MMAs of a k-block take to execute.
+        // Measured on one B200, warp-wide -> single lane: FP4 3470 -> 4200 TFLOPS, masked FP8 1009 -> 1052, split-K FP8
+        // at M = 128 2 to 7 % faster, the contiguous grouped GEMM 1842 -> 1994, FP8 on CTA pairs 154 -> 148 us (224 columns) and
+        // 222 -> 177 us (128) on 4096 x 7168 x 7168; BF16 on pairs unchanged.
         const bool issuer = elect_one();
         const uint32_t issuer_lane = (uint32_t)__ffs(__ballot_sync(0xffffffffu, issuer)) - 1u;
         uint32_t ok = 1;
@@ -521,77 +519,70 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             const uint32_t d_tmem = tmem + as * kAccStageCols;
             const uint32_t idesc = t.tail ? p.idesc_tail : p.idesc;   // operand formats, tile shape and majors, built by the host
             const uint32_t kb_first = SPLIT ? t.kb0 : 0u, kb_count = SPLIT ? t.kb1 - t.kb0 : p.num_k_blocks;
-            if (!kConsLane || issuer) {
+            if (issuer) {
             for (uint32_t ki = 0; ki < kb_count; ++ki) {
                 const uint32_t kb = kb_first + ki;
-                if (!(ok = kConsLane ? (uint32_t)mbar_wait(smem_u32(&bars->full[stage]), phase, wc, kWaitFull)
-                                     : (uint32_t)DG_WARP_WAIT(smem_u32(&bars->full[stage]), phase, wc, kWaitFull))) break;
+                if (!(ok = (uint32_t)mbar_wait(smem_u32(&bars->full[stage]), phase, wc, kWaitFull))) break;
                 if (kHasSf && (kb & p.sf_load_mask) == 0) {
                     // the SF warp has copied this k-block's scale factors into the other set (its commit arrives here)
-                    if (!(ok = kConsLane ? (uint32_t)mbar_wait(smem_u32(&bars->sf_ready[stage]), (sf_bits >> stage) & 1u, wc, kWaitSfReady)
-                                         : (uint32_t)DG_WARP_WAIT(smem_u32(&bars->sf_ready[stage]), (sf_bits >> stage) & 1u, wc, kWaitSfReady))) break;
+                    if (!(ok = (uint32_t)mbar_wait(smem_u32(&bars->sf_ready[stage]), (sf_bits >> stage) & 1u, wc, kWaitSfReady))) break;
                     sf_bits ^= 1u << stage;
                     if (SFW) sf_set ^= 1u;
                 }
                 tc_fence_after();
                 const uint32_t sa = stage_addr(stage);
                 const uint32_t sfa_col = tmem + sf_set_col(sf_set) + kSfaOff, sfb_col = tmem + sf_set_col(sf_set) + kSfbOff;
-                if (kConsLane || elect_one()) {
-                    if (kHasSf && !SFW && (kb & p.sf_load_mask) == 0) {
-                        // in order with the MMAs in the tensor pipe: the copy may overwrite the set the MMAs before it read
-                        copy_sf(sa, sf_set);
-                    }
-                    // K-major tile: 8-row groups 1024 B apart.  MN-major tile: 8 K rows of an atom are 1024 B
-                    // apart (SBO), atoms along MN box_bytes apart (LBO).
-                    const uint64_t a_desc = (MNM && p.a_mn) ? make_smem_desc(sa, 1024, p.box_bytes, kLayoutSw128) : make_kmajor_sw128_desc(sa);
-                    const uint64_t b_desc = (MNM && p.b_mn) ? make_smem_desc(sa + p.off_b, 1024, p.box_bytes, kLayoutSw128)
-                                                            : make_kmajor_sw128_desc(sa + p.off_b);
-                    const uint32_t a_step = (MNM && p.a_mn) ? p.mn_kstep : 2u, b_step = (MNM && p.b_mn) ? p.mn_kstep : 2u;
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) {
-                        // 32 bytes of K per MMA (32 FP8, 64 FP4, 16 BF16): +2 in the >>4 address field of a
-                        // K-major tile, that many whole K rows of 128 bytes in an MN-major one.
-                        const uint64_t ad = a_desc + a_step * k, bd = b_desc + b_step * k;
-                        const uint32_t acc = (ki | k) != 0u ? 1u : 0u;
-                        if (KIND == kBf16) {
-                            tc_mma_bf16<CL>(d_tmem, ad, bd, idesc, acc);
-                        } else if (KIND == kFp8) {
-                            // one SF byte per row per MMA: byte k of the word (gran 32), or the
-                            // byte of this k-block within its 512-wide SF row (gran 128)
-                            const uint32_t ida = p.sfa_shift == 0 ? k : (kb & 3u);
-                            const uint32_t idb = p.sfb_shift == 0 ? k : (kb & 3u);
-                            tc_mma_mxf8<CL>(d_tmem, ad, bd, idesc_with_sf_ids(idesc, ida, idb), acc, sfa_col, sfb_col);
-                        } else {
-                            // two SF bytes per row per MMA (64 elements): half-word (k & 1) of SF row (k >> 1)
-                            const uint32_t sub = k >> 1, id = (k & 1u) * 2u;
-                            tc_mma_mxf4<CL>(d_tmem, ad, bd, idesc_with_sf_ids(idesc, id, id), acc,
-                                            sfa_col + sub * 4u, sfb_col + sub * p.sfb_chunks * 4u);
-                        }
-                    }
-                    // free the stage in both CTAs / publish the accumulator to both epilogues (a pair: one commit
-                    // whose completion signal goes to the same barrier of both CTAs; 2 to 6 % faster than two commits)
-                    if (CL == 2) {
-                        tc_commit_pair(smem_u32(&bars->empty[stage]));
-                        if (ki + 1 == kb_count) tc_commit_pair(smem_u32(&bars->tmem_full[as]));
-                    } else {
-                        tc_commit<CL>(smem_u32(&bars->empty[stage]));
-                        if (ki + 1 == kb_count) tc_commit<CL>(smem_u32(&bars->tmem_full[as]));
-                    }
-                    // last k-block that reads this SF set: once its MMAs are through, the SF warp may overwrite the set
-                    if (kHasSf && SFW && (ki + 1 == kb_count || ((kb + 1u) & p.sf_load_mask) == 0)) tc_commit<CL>(smem_u32(&bars->sf_free[sf_set]));
+                if (kHasSf && !SFW && (kb & p.sf_load_mask) == 0) {
+                    // in order with the MMAs in the tensor pipe: the copy may overwrite the set the MMAs before it read
+                    copy_sf(sa, sf_set);
                 }
-                if (!kConsLane) __syncwarp();
+                // K-major tile: 8-row groups 1024 B apart.  MN-major tile: 8 K rows of an atom are 1024 B
+                // apart (SBO), atoms along MN box_bytes apart (LBO).
+                const uint64_t a_desc = (MNM && p.a_mn) ? make_smem_desc(sa, 1024, p.box_bytes, kLayoutSw128) : make_kmajor_sw128_desc(sa);
+                const uint64_t b_desc = (MNM && p.b_mn) ? make_smem_desc(sa + p.off_b, 1024, p.box_bytes, kLayoutSw128)
+                                                        : make_kmajor_sw128_desc(sa + p.off_b);
+                const uint32_t a_step = (MNM && p.a_mn) ? p.mn_kstep : 2u, b_step = (MNM && p.b_mn) ? p.mn_kstep : 2u;
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    // 32 bytes of K per MMA (32 FP8, 64 FP4, 16 BF16): +2 in the >>4 address field of a
+                    // K-major tile, that many whole K rows of 128 bytes in an MN-major one.
+                    const uint64_t ad = a_desc + a_step * k, bd = b_desc + b_step * k;
+                    const uint32_t acc = (ki | k) != 0u ? 1u : 0u;
+                    if (KIND == kBf16) {
+                        tc_mma_bf16<CL>(d_tmem, ad, bd, idesc, acc);
+                    } else if (KIND == kFp8) {
+                        // one SF byte per row per MMA: byte k of the word (gran 32), or the
+                        // byte of this k-block within its 512-wide SF row (gran 128)
+                        const uint32_t ida = p.sfa_shift == 0 ? k : (kb & 3u);
+                        const uint32_t idb = p.sfb_shift == 0 ? k : (kb & 3u);
+                        tc_mma_mxf8<CL>(d_tmem, ad, bd, idesc_with_sf_ids(idesc, ida, idb), acc, sfa_col, sfb_col);
+                    } else {
+                        // two SF bytes per row per MMA (64 elements): half-word (k & 1) of SF row (k >> 1)
+                        const uint32_t sub = k >> 1, id = (k & 1u) * 2u;
+                        tc_mma_mxf4<CL>(d_tmem, ad, bd, idesc_with_sf_ids(idesc, id, id), acc,
+                                        sfa_col + sub * 4u, sfb_col + sub * p.sfb_chunks * 4u);
+                    }
+                }
+                // free the stage in both CTAs / publish the accumulator to both epilogues (a pair: one commit
+                // whose completion signal goes to the same barrier of both CTAs; 2 to 6 % faster than two commits)
+                if (CL == 2) {
+                    tc_commit_pair(smem_u32(&bars->empty[stage]));
+                    if (ki + 1 == kb_count) tc_commit_pair(smem_u32(&bars->tmem_full[as]));
+                } else {
+                    tc_commit<CL>(smem_u32(&bars->empty[stage]));
+                    if (ki + 1 == kb_count) tc_commit<CL>(smem_u32(&bars->tmem_full[as]));
+                }
+                // last k-block that reads this SF set: once its MMAs are through, the SF warp may overwrite the set
+                if (kHasSf && SFW && (ki + 1 == kb_count || ((kb + 1u) & p.sf_load_mask) == 0)) tc_commit<CL>(smem_u32(&bars->sf_free[sf_set]));
                 if (++stage == p.num_stages) { stage = 0; phase ^= 1u; }
             }
             }
             __syncwarp();
-            if (kConsLane) {
-                ok = __shfl_sync(0xffffffffu, ok, issuer_lane);
-                stage = __shfl_sync(0xffffffffu, stage, issuer_lane);
-                phase = __shfl_sync(0xffffffffu, phase, issuer_lane);
-                sf_bits = __shfl_sync(0xffffffffu, sf_bits, issuer_lane);
-                sf_set = __shfl_sync(0xffffffffu, sf_set, issuer_lane);
-            }
+            ok = __shfl_sync(0xffffffffu, ok, issuer_lane);
+            stage = __shfl_sync(0xffffffffu, stage, issuer_lane);
+            phase = __shfl_sync(0xffffffffu, phase, issuer_lane);
+            sf_bits = __shfl_sync(0xffffffffu, sf_bits, issuer_lane);
+            sf_set = __shfl_sync(0xffffffffu, sf_set, issuer_lane);
         }
     } else if (warp == 2 && kHasSf) {
         // ===================================================== SF warp: transposes the SF rows in shared memory and copies them into tensor memory
@@ -1087,23 +1078,27 @@ static uint32_t pick_block_n(int kind, uint32_t m_tiles_total, uint32_t n, uint3
     return best;
 }
 
-// Dense FP8 with per-128 scales: tile shape from measured tile times.  A tile of kb k-blocks takes about
-// fixed + kb * per_kb nanoseconds (B200, 4096 x 7168 x {2048, 16384}, both modes; widths are multiples of 16, the 224-wide
-// single-CTA tile has four pipeline stages where 192 has five, hence its jump; a CTA pair takes the same
-// time per k-block at every width), and a launch takes waves x tile time.
-static void pick_dense_fp8_tile(uint32_t m, uint32_t groups, uint32_t n, uint32_t kb, uint32_t sms, uint32_t* cl_out, uint32_t* bn_out,
-                                bool pairs_allowed = true) {
-    static const uint32_t widths[8] = {64, 96, 128, 160, 176, 192, 208, 224};
-    static const double single_kb[8] = {214, 233, 273, 331, 355, 361, 394, 537};
-    static const double pair_kb[8] = {423, 417, 414, 392, 0, 442, 0, 447};   // 0: not measured, not offered
+// Block-scaled GEMMs: tile shape from measured tile times.  A tile of kb k-blocks takes about fixed + kb * per_kb
+// nanoseconds (B200, 4096 x 7168 x 7168 at every width in both modes, launches back to back, so at the clocks the power cap
+// leaves; widths are multiples of 16, the 224-wide single-CTA tile has four pipeline stages where 192 has five,
+// hence its jump), and a launch takes waves x tile time.  The pair's 224 columns are the fastest shape for whole waves
+// (147 us per 128, 154 us per 32, 78 us FP4; single CTAs at best 176, 179 and 86), single CTAs fit few tiles better.
+struct TileTimes { double single_kb[8], pair_kb[8]; };    // 0: not measured, not offered
+static const uint32_t kTileWidths[8] = {64, 96, 128, 160, 176, 192, 208, 224};
+static const TileTimes kFp8Per128 = {{181, 200, 248, 302, 331, 328, 369, 429}, {194, 210, 233, 277, 0, 302, 336, 367}};
+static const TileTimes kFp8Per32 = {{231, 228, 254, 322, 0, 344, 376, 441}, {0, 268, 279, 322, 0, 332, 363, 384}};    // either operand per 32
+static const TileTimes kFp4Times = {{214, 231, 254, 324, 0, 320, 354, 392}, {0, 303, 305, 363, 0, 364, 378, 385}};
+static void pick_scaled_tile(const TileTimes& times, uint32_t m, uint32_t groups, uint32_t n, uint32_t kb, uint32_t sms, uint32_t* cl_out,
+                             uint32_t* bn_out, bool pairs_allowed = true) {
     double best = 1e30;
     for (uint32_t cl = 1; cl <= ((m > kBlockM && pairs_allowed) ? 2u : 1u); ++cl) {
         for (uint32_t i = 0; i < 8; ++i) {
-            const uint32_t bn = widths[i];
-            if (cl == 2 && pair_kb[i] == 0) continue;
+            const uint32_t bn = kTileWidths[i];
+            const double per_kb = cl == 1 ? times.single_kb[i] : times.pair_kb[i];
+            if (per_kb == 0) continue;
             const uint64_t tiles = (uint64_t)groups * ceil_div(m, kBlockM * cl) * ceil_div(n, bn);
             const uint64_t waves = (tiles + sms / cl - 1) / (sms / cl);
-            const double cost = (double)waves * (cl == 1 ? 1300.0 + kb * single_kb[i] : 400.0 + kb * pair_kb[i]);
+            const double cost = (double)waves * ((cl == 1 ? 1300.0 : 400.0) + kb * per_kb);
             if (cost < best) { best = cost; *cl_out = cl; *bn_out = bn; }
         }
     }
@@ -1111,7 +1106,7 @@ static void pick_dense_fp8_tile(uint32_t m, uint32_t groups, uint32_t n, uint32_
 
 static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k, uint32_t num_groups,
                          uint32_t expected_m, uint32_t gran_a, uint32_t gran_b, const DeviceInfo* dev, Plan* plan,
-                         bool allow_dynamic = true, bool a_mn = false, bool b_mn = false) {
+                         bool allow_dynamic = true, bool a_mn = false, bool b_mn = false, bool plain = true) {
     note_env();
     GemmParams& p = plan->p;
     p = GemmParams{};
@@ -1123,13 +1118,15 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     // that share B.  In the contiguous grouped layout the kernel pairs neighbouring blocks of one
     // expert and runs an odd last block with an idle partner.
     const uint32_t rows_per_group = gtype == kMasked ? (expected_m ? expected_m : m) : m;
-    // Measured on B200: pairs win for FP8 / BF16 dense and masked GEMMs; FP4 (scale factors on
-    // every k-block, twice the UTCCP traffic) and the contiguous layout (an expert's weights are
-    // shared by only a few row blocks) run faster on single CTAs.
-    // With FP8 scale factors per 32 (copies into TMEM on every k-block, issued for both CTAs) pairs lose: 960 against
-    // 1570 TFLOPS on 4096 x 7168 x 16384.
-    const bool sf_every_block = kind == kFp8 && (gran_a == 32 || gran_b == 32);
-    uint32_t cl = (rows_per_group > kBlockM && kind != kFp4 && gtype != kContiguous && !sf_every_block) ? 2u : 1u;
+    // Dense and masked block-scaled GEMMs choose below, from measured tile times.  In the contiguous layout (FP8) an expert
+    // with an odd number of row blocks leaves half a pair idle, so pairs are for layouts of about two and a half blocks per
+    // expert or more (m counts the padding): 64 experts, N 4096 K 7168, 505 rows each 894 us on pairs against 971, 252
+    // rows 574 / 588 (N 7168 K 2048: 311 / 328 us).  Layouts sized for the worst case (a device-side block count,
+    // rows stored through addresses) say nothing about their rows and share their SMs with transfers: single CTAs and
+    // the dynamic schedule.
+    const bool pair_contiguous = gtype == kContiguous && kind == kFp8 && gran_a == 128 && gran_b == 128 && plain && n >= 224u &&
+                                 (uint64_t)m >= 320ull * num_groups;
+    uint32_t cl = (gtype == kContiguous ? pair_contiguous : rows_per_group > kBlockM) ? 2u : 1u;
     const uint32_t forced_cl = env_u32("DG_CLUSTER", 0);
     if (forced_cl == 1 || forced_cl == 2) cl = forced_cl;
     if (gtype == kContiguous && m / kBlockM > kMaxPairedBlocks) cl = 1;   // the in-kernel tile list is bounded
@@ -1137,13 +1134,15 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     // 128 columns, and two of them per CTA would be wider than the accumulators beside the scale factors.
     if ((a_mn || b_mn) && (kind != kBf16 || gtype != kNormal)) cl = 1;
     uint32_t dense_bn = 0;
-    if (kind == kFp8 && (gtype == kNormal || gtype == kMasked) && gran_a == 128 && gran_b == 128 && !a_mn && !b_mn &&
-        (gtype == kMasked || m > kBlockM) && forced_cl == 0 && env_u32("DG_BLOCK_N", 0) == 0)
-        pick_dense_fp8_tile(rows_per_group, gtype == kMasked ? num_groups : 1u, n, p.num_k_blocks, sms, &cl, &dense_bn);   // masked: expected rows per group
+    const TileTimes& times = kind == kFp4 ? kFp4Times : (gran_a == 128 && gran_b == 128) ? kFp8Per128 : kFp8Per32;
+    if (kind != kBf16 && (gtype == kNormal || gtype == kMasked) && !a_mn && !b_mn && (gtype == kMasked || m > kBlockM) &&
+        forced_cl == 0 && env_u32("DG_BLOCK_N", 0) == 0)
+        pick_scaled_tile(times, rows_per_group, gtype == kMasked ? num_groups : 1u, n, p.num_k_blocks, sms, &cl, &dense_bn);   // masked: expected rows per group
     // the contiguous grouped layout on single CTAs: the same table (208 columns and five stages for N = 4096: 1994
     // against 1849 TFLOPS on 224 columns and four)
     if (kind == kFp8 && gtype == kContiguous && cl == 1 && gran_a == 128 && gran_b == 128 && !a_mn && !b_mn && env_u32("DG_BLOCK_N", 0) == 0)
-        pick_dense_fp8_tile(m, 1u, n, p.num_k_blocks, sms, &cl, &dense_bn, false);
+        pick_scaled_tile(times, m, 1u, n, p.num_k_blocks, sms, &cl, &dense_bn, false);
+    if (pair_contiguous && cl == 2 && env_u32("DG_BLOCK_N", 0) == 0) dense_bn = 224u;   // the widest tile reads the least
     plan->cluster = cl;
     const uint32_t tile_m = kBlockM * cl;
     const uint32_t units = sms / cl;
@@ -1402,7 +1401,8 @@ static int32_t run_gemm(const dg_operand_t* a, const dg_operand_t* b, dg_output_
     DG_CUDA_CHECK(cudaStreamIsCapturing(s, &capturing));
     Plan plan;
     if ((st = make_plan(kind, gtype, m, n, k, num_groups, expected_m, gran_a, gran_b, dev, &plan,
-                        capturing == cudaStreamCaptureStatusNone, a_mn, b_mn)) != DG_OK) return st;
+                        capturing == cudaStreamCaptureStatusNone, a_mn, b_mn,
+                        !d_row_map && !d_row_ptr && !m_blocks_dev && !a_row_src)) != DG_OK) return st;
     GemmParams& p = plan.p;
     p.out_f32 = out->dtype == DG_F32;
     p.accumulate = accumulate ? 1u : 0u;

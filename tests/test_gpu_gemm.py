@@ -426,3 +426,39 @@ def test_config_introspection():
     assert cfg["smem_bytes"] <= 232448 and cfg["num_stages"] >= 2
     assert get_gemm_config(Dtype.Fp4, 0, 8192, 8192, 8192)["block_k"] == 256
     assert get_gemm_config(Dtype.Bf16, 0, 2048, 2048, 2048)["block_k"] == 64
+
+
+@pytest.mark.parametrize("groups,n,k,blocks", [
+    (2, 224, 512, [0, 0, 0, 1, 1]),                          # one full tile wide, 320 rows per group: the first size on pairs
+    (2, 224, 512, [0, 0, 1, 1]),                             # the last on single CTAs
+    (3, 1000, 1024, [2, 2, 2, -1, 0, 1, 1, -1, 2, 2]),       # narrow last column tile, odd runs, unowned blocks
+    (2, 220, 512, [0, 1, 1, 1, 0, 0]),                       # narrower than a tile: single CTAs
+])
+def test_m_grouped_contiguous_choice_of_pairs(groups, n, k, blocks):
+    """FP8 per-128: layouts of at least 320 rows per group and 224 columns run on CTA pairs with 224-wide tiles.  The result
+    is the same bit for bit as on single CTAs, and unowned blocks stay untouched."""
+    m = 128 * len(blocks)
+    a, ga = quantised_operand(randn((m, k), 21), "fp8", 128)
+    b, gb = _stacked_b("fp8", groups, n, k, 22, gran=128)
+    got = []
+    for cluster in (None, "1"):
+        if cluster:
+            os.environ["DG_CLUSTER"] = cluster
+        out = new_output(m, n, fill=3.0)
+        m_grouped_gemm_nt_contiguous(a, b, out, dev(np.array(blocks, dtype=np.int32)), groups)
+        poll_device_status()
+        got.append(to_f32(out))
+    assert np.array_equal(got[0], got[1])
+    for i, e in enumerate(blocks):
+        rows = np.arange(128 * i, 128 * (i + 1))
+        if e < 0:
+            assert (got[0][rows] == 3.0).all()
+        else:
+            assert_close_to_oracle(got[0][rows], bf16_round(o.gemm_ref(ga, gb, rows=rows, n=n, b_row0=e * n)), "fp8", f"block {i}")
+
+
+@pytest.mark.parametrize("kind,gran", [("fp8", 32), ("fp4", 32)])
+@pytest.mark.parametrize("m,n,k", [(129, 200, 768), (300, 1000, 2304), (512, 2560, 512)])
+def test_scale_factors_on_every_k_block_on_pairs(kind, gran, m, n, k):
+    """FP8 per-32 and FP4 with more than one row block run on CTA pairs: ragged rows, a second CTA with one row, narrow tiles."""
+    run_dense(kind, m, n, k, gran_a=gran, gran_b=gran, seed=m + n)
