@@ -101,7 +101,7 @@ struct MqaParams {
 
 struct __align__(8) MqaBarriers {
     uint64_t kv_full[kMqaMaxKvStages];
-    uint64_t kv_ready[kMqaMaxKvStages];   // ue8m0: scale factors in place
+    uint64_t kv_ready[kMqaMaxKvStages];   // ue8m0 over contiguous kv: scale factors in place
     uint64_t kv_empty[kMqaMaxKvStages];
     uint64_t q_full[2], q_ready[2], q_empty[2];
     uint64_t tmem_full[kDecStages], tmem_empty[kDecStages];   // two of them outside decode
@@ -252,8 +252,8 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     if (threadIdx.x == 0) {
         bars->abort = 0;
         for (uint32_t s = 0; s < p.kv_stages; ++s) {
-            mbar_init(smem_u32(&bars->kv_full[s]), 1);
-            mbar_init(smem_u32(&bars->kv_ready[s]), PAGED ? 32 : 1);   // paged: one arrival per lane of the SF warp
+            mbar_init(smem_u32(&bars->kv_full[s]), PAGED ? 33 : 1);    // paged: the producer, and one arrival per lane of the SF warp
+            mbar_init(smem_u32(&bars->kv_ready[s]), 1);
             mbar_init(smem_u32(&bars->kv_empty[s]), 1);
         }
         for (uint32_t s = 0; s < 2; ++s) {
@@ -391,7 +391,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     ok = wait_on(smem_u32(&bars->tmem_empty[s]), ((acc_bits >> s) & 1u) ^ 1u, kWaitTmemEmpty);
             for (uint32_t kb = k.kb0; ok && kb < k.kb1; ++kb) {
                 if (!(ok = wait_on(smem_u32(&bars->kv_full[stage]), phase, kWaitFull))) break;
-                if (SCALED && !(ok = wait_on(smem_u32(&bars->kv_ready[stage]), phase, kWaitSfReady))) break;
+                if (SCALED && !PAGED && !(ok = wait_on(smem_u32(&bars->kv_ready[stage]), phase, kWaitSfReady))) break;
                 if (PAGED) fence_proxy_async_smem();     // the scale words came by generic-proxy copies, tcgen05.cp reads them
                 const uint32_t kaddr = base + p.off_kv + stage * p.kv_stage_bytes;
                 const uint64_t kv_desc = make_smem_desc(kaddr, p.sbo, 0, p.layout);
@@ -473,7 +473,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             if (PAGED) {
                 // Lane l fetches the words of tokens 4 l .. 4 l + 3 of a block: they lie in one page (pages hold a
                 // multiple of four tokens), so it is one block-table entry.  The words are copied asynchronously, straight
-                // to their places in the stage, and the stage's barrier counts the lanes' copies: as many blocks are under
+                // to their places in the stage, and the stage's barrier counts the lanes' copies beside the kv rows: as many blocks are under
                 // way as the ring has stages.  (Held in registers two blocks ahead, a load's trip to memory every two
                 // blocks bounded decode: 690 ns per block.)  The block-table entries run eight blocks ahead in
                 // registers that are not touched before their block comes up; the loop is unrolled for that.
@@ -500,7 +500,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         const uint32_t sf = base + p.off_kv + stage * p.kv_stage_bytes + p.kv_sf_off + (lane >> 3) * 4u;
 #pragma unroll
                         for (uint32_t i = 0; i < 4; ++i) cp_async_4(sf + 16u * ((4u * lane + i) & 31u), p.kv_sf + row + i);
-                        cp_async_arrive(smem_u32(&bars->kv_ready[stage]));
+                        cp_async_arrive(smem_u32(&bars->kv_full[stage]));
                         if (++stage == p.kv_stages) { stage = 0; phase ^= 1u; }
                     }
                 }
