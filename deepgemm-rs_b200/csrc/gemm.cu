@@ -1118,14 +1118,15 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     // that share B.  In the contiguous grouped layout the kernel pairs neighbouring blocks of one
     // expert and runs an odd last block with an idle partner.
     const uint32_t rows_per_group = gtype == kMasked ? (expected_m ? expected_m : m) : m;
-    // Dense and masked block-scaled GEMMs choose below, from measured tile times.  In the contiguous layout (FP8) an expert
-    // with an odd number of row blocks leaves half a pair idle, so pairs are for layouts of about two and a half blocks per
-    // expert or more (m counts the padding): 64 experts, N 4096 K 7168, 505 rows each 894 us on pairs against 971, 252
-    // rows 574 / 588 (N 7168 K 2048: 311 / 328 us).  Layouts sized for the worst case (a device-side block count,
-    // rows stored through addresses) say nothing about their rows and share their SMs with transfers: single CTAs and
-    // the dynamic schedule.
+    // Dense, masked and batched block-scaled GEMMs choose below, from measured tile times.  In the contiguous layout (FP8) an
+    // expert with an odd number of row blocks leaves half a pair idle, and that half costs time and energy: with four
+    // and a half blocks per expert (256 experts, N 4096 K 7168, 512 rows each) a MoE step on pairs is 7 % faster in a
+    // burst but 4 % slower under lasting load at the power cap.  So pairs are for layouts of eight blocks per
+    // expert or more (m counts the padding).  Layouts sized for the worst case (a device-side block count, rows stored
+    // through addresses) say nothing about their rows and share their SMs with transfers: single CTAs and the
+    // dynamic schedule.
     const bool pair_contiguous = gtype == kContiguous && kind == kFp8 && gran_a == 128 && gran_b == 128 && plain && n >= 224u &&
-                                 (uint64_t)m >= 320ull * num_groups;
+                                 (uint64_t)m >= 1088ull * num_groups;
     uint32_t cl = (gtype == kContiguous ? pair_contiguous : rows_per_group > kBlockM) ? 2u : 1u;
     const uint32_t forced_cl = env_u32("DG_CLUSTER", 0);
     if (forced_cl == 1 || forced_cl == 2) cl = forced_cl;
@@ -1135,9 +1136,9 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     if ((a_mn || b_mn) && (kind != kBf16 || gtype != kNormal)) cl = 1;
     uint32_t dense_bn = 0;
     const TileTimes& times = kind == kFp4 ? kFp4Times : (gran_a == 128 && gran_b == 128) ? kFp8Per128 : kFp8Per32;
-    if (kind != kBf16 && (gtype == kNormal || gtype == kMasked) && !a_mn && !b_mn && (gtype == kMasked || m > kBlockM) &&
-        forced_cl == 0 && env_u32("DG_BLOCK_N", 0) == 0)
-        pick_scaled_tile(times, rows_per_group, gtype == kMasked ? num_groups : 1u, n, p.num_k_blocks, sms, &cl, &dense_bn);   // masked: expected rows per group
+    if (kind != kBf16 && gtype != kContiguous && !a_mn && !b_mn && (gtype == kMasked || m > kBlockM) && forced_cl == 0 &&
+        env_u32("DG_BLOCK_N", 0) == 0)
+        pick_scaled_tile(times, rows_per_group, gtype == kNormal ? 1u : num_groups, n, p.num_k_blocks, sms, &cl, &dense_bn);   // masked: expected rows per group
     // the contiguous grouped layout on single CTAs: the same table (208 columns and five stages for N = 4096: 1994
     // against 1849 TFLOPS on 224 columns and four)
     if (kind == kFp8 && gtype == kContiguous && cl == 1 && gran_a == 128 && gran_b == 128 && !a_mn && !b_mn && env_u32("DG_BLOCK_N", 0) == 0)
@@ -1198,12 +1199,10 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     p.sfa_shift = gran_a == 128 ? 2u : 0u;
     p.sfb_shift = gran_b == 128 ? 2u : 0u;
     p.sf_load_mask = (gran_a == 128 && gran_b == 128) ? 3u : 0u;
-    // Who copies the SF rows into tensor memory (tcgen05.cp, some 200 cycles of issue time each).  FP8 with per-128
-    // scales on single CTAs: the SF warp, which takes the copies off the MMA issuer's loop (grouped GEMM 1710 ->
-    // 1776 TFLOPS, M = 128 shapes 2 to 4 % faster).  SF on every k-block (FP4, per-32 FP8): the SF warp's own loop
-    // (transposition + up to six copies) then becomes the limit, the MMA issuer keeps the copies.  CTA pairs: the
-    // MMA issuer as well (dense FP8 2411 against 2317 TFLOPS).  The choice is a template parameter: as a run-time
-    // branch in the k-loop it cost the pair kernel 13 %.
+    // Who copies the SF rows into tensor memory (tcgen05.cp).  FP8 with per-128 scales on single CTAs: the SF warp, which
+    // takes the copies off the MMA issuer's loop (grouped GEMM 1710 -> 1776 TFLOPS, M = 128 shapes 2 to 4 % faster when
+    // that was built).  SF on every k-block (FP4, per-32 FP8): the MMA issuer, in order with its MMAs (one SF warp, or
+    // two taking turns, were slower: FP4 105 -> 163 us).  CTA pairs: the MMA issuer as well.
     p.sf_cp_by_mma = env_u32("DG_SF_CP_BY_MMA", p.sf_load_mask == 0 ? 1u : 0u);
     // per CTA; a K-major tile holds its rows x 128 bytes of K, an MN-major one whole atoms of 128 bytes x BLOCK_K rows
     const uint32_t block_k_rows = kind == kBf16 ? 64u : 128u;
