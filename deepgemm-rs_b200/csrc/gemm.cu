@@ -1119,14 +1119,15 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     // expert and runs an odd last block with an idle partner.
     const uint32_t rows_per_group = gtype == kMasked ? (expected_m ? expected_m : m) : m;
     // Dense, masked and batched block-scaled GEMMs choose below, from measured tile times.  In the contiguous layout (FP8) an
-    // expert with an odd number of row blocks leaves half a pair idle, and that half costs time and energy: with four
-    // and a half blocks per expert (256 experts, N 4096 K 7168, 512 rows each) a MoE step on pairs is 7 % faster in a
-    // burst but 4 % slower under lasting load at the power cap.  So pairs are for layouts of eight blocks per
-    // expert or more (m counts the padding).  Layouts sized for the worst case (a device-side block count, rows stored
+    // expert with an odd number of row blocks leaves half a pair idle, which costs time and energy.  Measured under
+    // lasting load, single CTAs / pairs (m counts the padding): 64 experts of 252 rows (m 24320) a whole feed-forward layer 1210 /
+    // 1165 us, 512 rows (m 40960) the GEMM 1105 / 1040 us, 32 experts of 1024 rows 968 / 884 us; but 256 experts of 512 rows
+    // (m 163584) a whole step 4990 / 5340 us.  So pairs are for layouts of about two and a half blocks per expert or more,
+    // beyond 65536 rows of eight blocks or more.  Layouts sized for the worst case (a device-side block count, rows stored
     // through addresses) say nothing about their rows and share their SMs with transfers: single CTAs and the
     // dynamic schedule.
     const bool pair_contiguous = gtype == kContiguous && kind == kFp8 && gran_a == 128 && gran_b == 128 && plain && n >= 224u &&
-                                 (uint64_t)m >= 1088ull * num_groups;
+                                 (uint64_t)m >= (m <= 65536u ? 320ull : 1088ull) * num_groups;
     uint32_t cl = (gtype == kContiguous ? pair_contiguous : rows_per_group > kBlockM) ? 2u : 1u;
     const uint32_t forced_cl = env_u32("DG_CLUSTER", 0);
     if (forced_cl == 1 || forced_cl == 2) cl = forced_cl;

@@ -429,13 +429,13 @@ def test_config_introspection():
 
 
 @pytest.mark.parametrize("groups,n,k,blocks", [
-    (2, 224, 512, [0] * 8 + [1] * 9),                        # one full tile wide, 1088 rows per group: the first size on pairs
-    (2, 224, 512, [0] * 8 + [1] * 8),                        # the last on single CTAs
+    (2, 224, 512, [0, 0, 0, 1, 1]),                          # one full tile wide, 320 rows per group: the first size on pairs
+    (2, 224, 512, [0, 0, 1, 1]),                             # the last on single CTAs
     (1, 1000, 1024, [0, 0, 0, -1, 0, 0, -1, 0, 0]),          # narrow last column tile, odd runs, unowned blocks
     (1, 220, 512, [0] * 9),                                  # narrower than a tile: single CTAs
 ])
 def test_m_grouped_contiguous_choice_of_pairs(groups, n, k, blocks):
-    """FP8 per-128: layouts of at least 1088 rows per group and 224 columns run on CTA pairs with 224-wide tiles.  The result
+    """FP8 per-128: layouts of at least 320 rows per group and 224 columns run on CTA pairs with 224-wide tiles.  The result
     is the same bit for bit as on single CTAs, and unowned blocks stay untouched."""
     m = 128 * len(blocks)
     a, ga = quantised_operand(randn((m, k), 21), "fp8", 128)
