@@ -60,8 +60,10 @@ static_assert(mqa_launch_regs(8) == 168 && mqa_epilogue_regs(8) == 232, "registe
 constexpr uint32_t kDecStages = 6;         // decode: accumulator stages at most
 constexpr uint32_t kDecAccCols = 384;      // decode: columns they share
 constexpr uint32_t kDecArrivals = 48;      // decode: arrivals that free a stage, split evenly over its 4 nq reducing warps (nq <= 4)
-__host__ __device__ constexpr uint32_t dec_block_q(uint32_t heads) { return heads == 64 ? 3u : 4u; }   // queries of a request per task
-constexpr uint32_t kPagesAhead = 8;        // paged: block-table look-ups run so many kv blocks ahead
+constexpr uint32_t kDecBlockQ = 4;         // decode: queries of a request per task
+// paged: block-table look-ups run so many kv blocks ahead (64 heads, 128 requests x 1 token over up to 8192: 30.4 us with
+// eight, 27.9 with four, the same over 32768; the decode form the other way round, 83.6 / 85.1 us over 32768)
+__host__ __device__ constexpr uint32_t pages_ahead(bool dec) { return dec ? 8u : 4u; }
 constexpr uint32_t kMqaSfaCol = 448;       // ue8m0 contracts only: the accumulators are <= 192 wide
 constexpr uint32_t kMqaSfbCol = 452;
 
@@ -226,10 +228,12 @@ __device__ __forceinline__ float relu_nan(float x) {
 // U4: head counts that are not a multiple of 16 (their 4-column reduction loop is a variant of its own: as a
 // run-time branch beside the 16-column loop it cost the common case 4 %).
 // QPW: queries per warpgroup of the NUN variants (their NUN units are QPW queries of 16 * NUN / QPW heads).
-// DEC (paged, 32 or 64 heads): decode.  A request has one to four tokens, so with one warpgroup per query of the block
-// most warpgroups had nothing to reduce and the live ones ran at the latency of their TMEM loads.  Here the four
+// DEC (paged, 32 heads): decode.  A request has one to four tokens, so with two queries per warpgroup most warpgroups
+// had nothing to reduce and the live ones ran at the latency of their TMEM loads.  Here the four
 // warpgroups take (query, kv block) pairs: with nq queries in a task, 4 / nq kv blocks are reduced side by side, the
 // MMAs are only nq queries wide and the accumulator ring has as many stages as then fit in kDecAccCols columns.
+// (128 requests x 2 tokens over up to 32768: 103 -> 83 us.  64 heads are as fast without it for one or two tokens, 101.5 /
+// 101.3 us, and slower with it for three, 41.2 / 36.1 us over up to 8192: they keep one query per warpgroup.)
 // NUN: 16-column units a warpgroup reduces per kv block when that is known at compile time (4 / 8 = one query of
 // 64 / 128 heads per warpgroup: the unit loop is then straight-line code without counters), 0 = any.
 template <bool SCALED, bool FP4, bool PAGED, bool U4 = false, uint32_t NUN = 0, uint32_t QPW = 1, bool DEC = false>
@@ -248,6 +252,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const WaitCtx wc{p.status, &bars->abort};
     const uint32_t ep_warps = 4u * p.ep_groups;
+    constexpr uint32_t kAhead = pages_ahead(DEC);
 
     if (threadIdx.x == 0) {
         bars->abort = 0;
@@ -306,7 +311,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             __syncwarp();
             if (PAGED) {
                 // A block of 128 tokens is a run of whole pages (or half / a quarter of a large page): lane i looks up
-                // the page of box i in the block table.  The look-ups run eight blocks ahead of the loads, and the
+                // the page of box i in the block table.  The look-ups run some blocks ahead of the loads, and the
                 // loop is unrolled so that an entry stays in its register, untouched, until its block comes
                 // up: looked up inside the loop, each block cost the producer a trip to memory, and decode ran at
                 // that latency instead of the cache's bandwidth.
@@ -317,12 +322,12 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     const uint32_t pg = tok_of(kbx) >> page_shift;
                     return (kbx < k.kb1 && lane < p.boxes_per_block && pg < p.block_table_stride) ? __ldg(trow + pg) : 0u;
                 };
-                uint32_t pq[kPagesAhead];
+                uint32_t pq[kAhead];
 #pragma unroll
-                for (uint32_t j = 0; j < kPagesAhead; ++j) pq[j] = page_of(k.kb0 + j);
-                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kPagesAhead) {
+                for (uint32_t j = 0; j < kAhead; ++j) pq[j] = page_of(k.kb0 + j);
+                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kAhead) {
 #pragma unroll
-                    for (uint32_t j = 0; j < kPagesAhead; ++j) {
+                    for (uint32_t j = 0; j < kAhead; ++j) {
                         const uint32_t kb = kb0 + j;
                         if (kb >= k.kb1) break;
                         if (!(ok = DG_WARP_WAIT(smem_u32(&bars->kv_empty[stage]), phase ^ 1u, wc, kWaitEmpty))) break;
@@ -331,7 +336,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         // rows past the table's width or pages outside the cache read row 0 (paged_row)
                         uint32_t row = pq[j] * p.page_kv + (tok_of(kb) & (p.page_kv - 1u));
                         if (row + p.box_rows > p.num_kv) row = 0u;
-                        pq[j] = page_of(kb + kPagesAhead);
+                        pq[j] = page_of(kb + kAhead);
                         if (lane == 0) mbar_arrive_expect_tx(bar, kv_tx);
                         __syncwarp();
                         if (lane < p.boxes_per_block) tma_load_2d(&tm_kv, bar, dst + lane * p.box_rows * p.row_bytes, 0, (int32_t)row);
@@ -475,7 +480,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 // multiple of four tokens), so it is one block-table entry.  The words are copied asynchronously, straight
                 // to their places in the stage, and the stage's barrier counts the lanes' copies beside the kv rows: as many blocks are under
                 // way as the ring has stages.  (Held in registers two blocks ahead, a load's trip to memory every two
-                // blocks bounded decode: 690 ns per block.)  The block-table entries run eight blocks ahead in
+                // blocks bounded decode: 690 ns per block.)  The block-table entries run some blocks ahead in
                 // registers that are not touched before their block comes up; the loop is unrolled for that.
                 const uint32_t* trow = p.block_table + (size_t)k.table_row * p.block_table_stride;
                 const uint32_t page_shift = (uint32_t)__ffs((int)p.page_kv) - 1u;
@@ -483,19 +488,19 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     const uint32_t pg = (kbx * kMqaBlockKv + 4u * lane) >> page_shift;
                     return (kbx < k.kb1 && pg < p.block_table_stride) ? __ldg(trow + pg) : 0u;
                 };
-                uint32_t pq[kPagesAhead];
+                uint32_t pq[kAhead];
 #pragma unroll
-                for (uint32_t j = 0; j < kPagesAhead; ++j) pq[j] = page_of(k.kb0 + j);
-                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kPagesAhead) {
+                for (uint32_t j = 0; j < kAhead; ++j) pq[j] = page_of(k.kb0 + j);
+                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kAhead) {
 #pragma unroll
-                    for (uint32_t j = 0; j < kPagesAhead; ++j) {
+                    for (uint32_t j = 0; j < kAhead; ++j) {
                         const uint32_t kb = kb0 + j;
                         if (kb >= k.kb1) break;
                         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->kv_empty[stage]), phase ^ 1u, wc, kWaitEmpty));
                         if (!ok) break;
                         uint32_t row = pq[j] * p.page_kv + ((kb * kMqaBlockKv + 4u * lane) & (p.page_kv - 1u));
                         if (row + 4u > p.num_kv) row = 0u;       // tokens past the table or the cache: masked by the epilogue
-                        pq[j] = page_of(kb + kPagesAhead);
+                        pq[j] = page_of(kb + kAhead);
                         // row r = 4 l + i of the block goes to position 4 (r % 32) + r / 32
                         const uint32_t sf = base + p.off_kv + stage * p.kv_stage_bytes + p.kv_sf_off + (lane >> 3) * 4u;
 #pragma unroll
@@ -657,6 +662,21 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         wp[2 * i + 1] = pack_f32x2(w4.z, w4.w);
                     }
                     uint32_t j = k.kb0 * kMqaBlockKv + quarter * 32u + lane;
+                    // A warpgroup none of whose queries the task has (decode: one or two tokens of a request in a block
+                    // of three) only hands the accumulator stages back; its issue slots go to the others.
+                    // (A loop of its own: as a branch inside the reduction loop below it cost that loop 17 %.)
+                    if (PAGED && q_first >= k.nq) {
+                        for (uint32_t kb = k.kb0; kb < k.kb1; ++kb) {
+                            const uint32_t as = acount & 1u, aphase = (acount >> 1) & 1u;
+                            ++acount;
+                            ok = __all_sync(0xffffffffu, mbar_wait(full0 + as * 8u, aphase, wc, kWaitTmemFull));
+                            if (!ok) break;
+                            tc_fence_after();
+                            tc_fence_before();
+                            if (lane == 0) mbar_arrive(empty0 + as * 8u);
+                        }
+                        continue;
+                    }
                     for (uint32_t kb = k.kb0; kb < k.kb1; ++kb, j += kMqaBlockKv) {
                         const uint32_t as = acount & 1u, aphase = (acount >> 1) & 1u;
                         ++acount;
@@ -912,8 +932,8 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
     // heads or two of 32 each): with two queries the MMAs are 128 columns wide and only eight warps reduce.
     const bool three_groups = SCALED && ((num_heads == 64 && block_q == 3) || (num_heads == 32 && block_q == 6));
     // decode: one to four tokens of a request, four warpgroups over (query, kv block) pairs
-    const bool dec = PAGED && (num_heads == 64 || num_heads == 32);
-    if (dec) block_q = dec_block_q(num_heads);
+    const bool dec = PAGED && num_heads == 32;
+    if (dec) block_q = kDecBlockQ;
     else if (three_groups) { /* keep */ }
     else if (block_q >= 4) block_q &= ~3u;
     else if (block_q == 3) block_q = 2;
@@ -1099,14 +1119,15 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
     };
     e = cudaSuccess;
     bool done = false;
-    if constexpr (PAGED) {
+    if (num_heads == 64 && p.block_q == p.ep_groups) {
+        done = true;
+        run(mqa_logits_kernel<SCALED, FP4, PAGED, false, 4>, 4);                                          // one query of 64 heads per warpgroup
+    } else if constexpr (PAGED) {
         done = dec;
-        if (dec && num_heads == 64) run(mqa_logits_kernel<SCALED, FP4, true, false, 4, 1, true>, 4);
-        else if (dec) run(mqa_logits_kernel<SCALED, FP4, true, false, 2, 1, true>, 4);
+        if (dec) run(mqa_logits_kernel<SCALED, FP4, true, false, 2, 1, true>, 4);
     } else {
-        done = (num_heads == 32 && p.block_q == 2u * p.ep_groups && p.ep_groups >= 3u) || (num_heads == 64 && p.block_q == p.ep_groups);
-        if (done && num_heads == 32) run(mqa_logits_kernel<SCALED, FP4, false, false, 4, 2>, 4);     // two queries of 32 heads per warpgroup
-        else if (done) run(mqa_logits_kernel<SCALED, FP4, false, false, 4>, 4);                      // one query of 64 heads per warpgroup
+        done = num_heads == 32 && p.block_q == 2u * p.ep_groups && p.ep_groups >= 3u;
+        if (done) run(mqa_logits_kernel<SCALED, FP4, false, false, 4, 2>, 4);                             // two queries of 32 heads per warpgroup
     }
     if (!done) {
         if (p.unit == 4u) run(mqa_logits_kernel<SCALED, FP4, PAGED, true>, 0);

@@ -235,3 +235,39 @@ def test_mqa_logits_paged_many_requests(kind, H, page_kv):
                 ref = (torch.relu(q_t[t] @ kv_t[torch.from_numpy(perm[r].astype(np.int64)).cuda()].reshape(-1, D)[:ctx[t]].T) * w_t[t][:, None]).sum(0)
                 err = (logits[t, :ctx[t]].float() - ref).abs().max() / ref.pow(2).mean().sqrt().clamp_min(1e-6)
                 assert err.item() <= 0.05
+
+
+@pytest.mark.parametrize("kind,H,page_kv", [("fp8", 64, 64), ("fp4", 64, 16)])
+def test_mqa_logits_paged_wide_requests(kind, H, page_kv):
+    """Requests of three to fourteen tokens: several query blocks per request, full ones and remainders, every logit
+    against the oracle."""
+    from deepgemm import mqa_logits_paged
+    rng = np.random.default_rng(H)
+    D, odt, dt = 128, *((o.FP8, Dtype.Fp8) if kind == "fp8" else (o.FP4, Dtype.Fp4))
+    ntok = np.array([3, 14, 4, 5, 6, 7, 12, 1, 13, 6, 2])
+    ctx_last = np.array([300, 700, 64, 129, 640, 7, 385, 512, 900, 31, 256])
+    nreq, T, per = len(ntok), int(ntok.sum()), -(-900 // page_kv)
+    rows = nreq * per * page_kv
+    codes, words = o.quant_mx_host(randn((rows, D), 8), odt, 32)
+    kvd = o.dequant_mx_host(codes, words, rows, D, odt, 32).reshape(-1, page_kv, D)
+    perm = rng.permutation(nreq * per).astype(np.int32).reshape(nreq, per)
+    first = np.concatenate([[0], np.cumsum(ntok)[:-1]])
+    table = np.zeros((T, per), dtype=np.int32)
+    table[first] = perm
+    ctx = np.concatenate([np.maximum(0, c - (n - 1 - np.arange(n))) for n, c in zip(ntok, ctx_last)]).astype(np.int32)
+    qc, qsf = o.quant_mx_host(randn((T * H, D), 9), odt, 32)
+    qd = o.dequant_mx_host(qc, qsf, T * H, D, odt, 32).reshape(T, H, D)
+    wb = torch.from_numpy(randn((T, H), 10)).to(torch.bfloat16)
+    width, fill = 904, -5.0
+    logits = torch.full((T, width), fill, dtype=torch.bfloat16, device="cuda")
+    qop = Operand.k_major(dt, T * H, D, D, sf_tensor(qsf, 32), dev(qc))
+    mqa_logits_paged(qop, dev(codes), dev(words[0, :rows].view(np.int32)), wb.cuda(), page_kv, nreq * per, dev(ctx),
+                     dev(np.repeat(np.arange(nreq, dtype=np.int32), ntok)), dev(table), per, T, H, D, logits, width)
+    poll_device_status()
+    got = logits.float().cpu().numpy()
+    for r in range(nreq):
+        t = slice(first[r], first[r] + ntok[r])
+        c = ctx[t].astype(np.uint32)
+        ref = o.mqa_logits_ref(qd[t], kvd[perm[r]].reshape(-1, D)[:c.max()], wb.float().numpy()[t], np.zeros(len(c), np.uint32), c)
+        ref = np.pad(ref, ((0, 0), (0, width - ref.shape[1])))
+        _check(got[t], o.bf16_bits_to_f32(o.f32_to_bf16_bits_np(ref)), np.zeros(len(c), np.uint32), c, width, fill)
