@@ -40,6 +40,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 namespace dg {
 
@@ -59,8 +60,11 @@ static_assert(mqa_launch_regs(4) == 96 && mqa_epilogue_regs(4) == 104, "register
 static_assert(mqa_launch_regs(8) == 168 && mqa_epilogue_regs(8) == 232, "register budget of the 128-head variant");
 constexpr uint32_t kDecStages = 6;         // decode: accumulator stages at most
 constexpr uint32_t kDecAccCols = 384;      // decode: columns they share
-constexpr uint32_t kDecArrivals = 48;      // decode: arrivals that free a stage, split evenly over its 4 nq reducing warps (nq <= 4)
-constexpr uint32_t kDecBlockQ = 4;         // decode: queries of a request per task
+constexpr uint32_t kDecArrivals = 48;      // decode: arrivals that free a stage, split evenly over its reducing warps (4, 8, 12 or 16)
+constexpr uint32_t kDecBlockQ = 6;         // decode: queries of a request per task
+// decode: queries the MMAs and the accumulator stages of a task are wide (nq rounded up: four widths, each with loops of its own)
+__host__ __device__ constexpr uint32_t dec_width_q(uint32_t nq) { return nq <= 2u ? nq : nq <= 4u ? 4u : 6u; }
+__host__ __device__ constexpr uint32_t dec_stages(uint32_t width) { return kDecAccCols / width < kDecStages ? kDecAccCols / width : kDecStages; }
 // paged: block-table look-ups run so many kv blocks ahead (64 heads, 128 requests x 1 token over up to 8192: 30.4 us with
 // eight, 27.9 with four, the same over 32768; the decode form the other way round, 83.6 / 85.1 us over 32768)
 __host__ __device__ constexpr uint32_t pages_ahead(bool dec) { return dec ? 8u : 4u; }
@@ -230,8 +234,10 @@ __device__ __forceinline__ float relu_nan(float x) {
 // QPW: queries per warpgroup of the NUN variants (their NUN units are QPW queries of 16 * NUN / QPW heads).
 // DEC (paged, 32 heads): decode.  A request has one to four tokens, so with two queries per warpgroup most warpgroups
 // had nothing to reduce and the live ones ran at the latency of their TMEM loads.  Here the four
-// warpgroups take (query, kv block) pairs: with nq queries in a task, 4 / nq kv blocks are reduced side by side, the
-// MMAs are only nq queries wide and the accumulator ring has as many stages as then fit in kDecAccCols columns.
+// warpgroups take (query, kv block) pairs: with nq <= 4 queries in a task, 4 / nq kv blocks are reduced side by side, the
+// MMAs are only as wide as the queries need and the accumulator ring has as many stages as then fit in kDecAccCols
+// columns.  Five or six queries go to three warpgroups, two each (with four per task at most, requests of five and six
+// tokens read their cache twice: 64 requests x 6 tokens over up to 8192 took 33.2 us instead of 26.4).
 // (128 requests x 2 tokens over up to 32768: 103 -> 83 us.  64 heads are as fast without it for one or two tokens, 101.5 /
 // 101.3 us, and slower with it for three, 41.2 / 36.1 us over up to 8192: they keep one query per warpgroup.)
 // NUN: 16-column units a warpgroup reduces per kv block when that is known at compile time (4 / 8 = one query of
@@ -386,10 +392,15 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 return kLaneLoop ? mbar_wait(bar, parity, wc, site) : (bool)DG_WARP_WAIT(bar, parity, wc, site);
             };
             if (!kLaneLoop || issuer) {
+            // WQ (DEC): queries the accumulator stages of this task are wide, a constant of the loop: with a run-time width
+            // the descriptor and the stage's column had to be moved to uniform registers for every MMA, and wide tasks ran
+            // at that pace (128 requests x 2 tokens over up to 32768: 82.6 us, with constants 72.8)
+            auto kv_loop = [&](auto width_q) {
+            constexpr uint32_t WQ = decltype(width_q)::value;
             // DEC: width and number of the accumulator stages of this task; the ring starts over at its first stage once
             // every stage of the task before (of another width, maybe) has been drained
-            const uint32_t dec_width = k.nq * p.num_heads, dec_stages = DEC ? min(kDecStages, kDecAccCols / dec_width) : 0u;
-            const uint32_t idesc = DEC ? make_idesc_bs(FP4 ? 1u : 0u, FP4 ? 1u : 0u, kMqaBlockKv, dec_width) : p.idesc;
+            constexpr uint32_t kWidth = WQ * 16u * NUN, kStages = WQ ? dec_stages(kWidth ? kWidth : 1u) : 0u;
+            const uint32_t idesc = DEC ? make_idesc_bs(FP4 ? 1u : 0u, FP4 ? 1u : 0u, kMqaBlockKv, kWidth) : p.idesc;
             uint32_t ring = 0;
             if (DEC)
                 for (uint32_t s = 0; ok && s < kDecStages; ++s)
@@ -404,11 +415,11 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 ++acount;
                 if (DEC) {
                     acc_bits ^= 1u << ring;
-                    if (++ring == dec_stages) ring = 0;
+                    if (++ring == kStages) ring = 0;
                 }
                 if (!(ok = wait_on(smem_u32(&bars->tmem_empty[as]), aphase ^ 1u, kWaitTmemEmpty))) break;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem + as * (DEC ? dec_width : acc_stride);
+                const uint32_t d_tmem = tmem + as * (DEC ? kWidth : acc_stride);
                 if (kLaneLoop || elect_one()) {
                     if (SCALED) {
                         if (!q_sf_copied)    // the q scales of this task: in order behind every MMA that used the previous task's
@@ -439,6 +450,12 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 q_sf_copied = true;
                 if (++stage == p.kv_stages) { stage = 0; phase ^= 1u; }
             }
+            };
+            if constexpr (!DEC) kv_loop(std::integral_constant<uint32_t, 0>{});
+            else if (k.nq == 1u) kv_loop(std::integral_constant<uint32_t, 1>{});
+            else if (k.nq == 2u) kv_loop(std::integral_constant<uint32_t, 2>{});
+            else if (k.nq <= 4u) kv_loop(std::integral_constant<uint32_t, 4>{});
+            else kv_loop(std::integral_constant<uint32_t, 6>{});
             }
             if (kLaneLoop) {
                 // the other lanes take over the issuer's position in the rings
@@ -583,13 +600,71 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 if (lane == 0) mbar_arrive(smem_u32(&bars->w_full[wb]));
                 ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->w_full[wb]), wphase, wc, kWaitWeights));
                 if (!ok) break;
+                if (DEC && k.nq > 4u) {
+                    // Two queries per warpgroup, three warpgroups, two accumulator stages in turn; the fourth warpgroup only
+                    // keeps count of their uses.
+                    constexpr uint32_t kStages = dec_stages(kDecBlockQ * 16u * (NUN ? NUN : 1u));
+                    static_assert(!DEC || kStages == 2u, "stages in turn");
+                    const uint32_t blocks = k.kb1 - k.kb0;
+                    if (wg < 3u) {
+                        const uint32_t qi = 2u * wg;
+                        const uint32_t s0 = win[qi], e0 = win[16u + qi], s1 = win[qi + 1u], e1 = win[17u + qi];   // e = 0: no such query
+                        const uint32_t span0 = e0 > s0 ? e0 - s0 : 0u, span1 = e1 > s1 ? e1 - s1 : 0u;
+                        __nv_bfloat16* const out = reinterpret_cast<__nv_bfloat16*>(p.logits) + (size_t)(k.q0 + qi) * p.logits_stride;
+                        const uint32_t lane_base = tmem + ((quarter * 32u) << 16) + qi * 16u * NUN;
+                        uint64_t wp[NUN ? 16u * NUN : 1u];
+#pragma unroll
+                        for (uint32_t i = 0; i < 8u * NUN; ++i) {
+                            const float4 w4 = reinterpret_cast<const float4*>(w + qi * 16u * NUN)[i];
+                            wp[2 * i] = pack_f32x2(w4.x, w4.y);
+                            wp[2 * i + 1] = pack_f32x2(w4.z, w4.w);
+                        }
+                        uint32_t j = k.kb0 * kMqaBlockKv + quarter * 32u + lane;
+                        for (uint32_t b = 0; b < blocks; ++b, j += kMqaBlockKv) {
+                            const uint32_t as = b & 1u;
+                            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->tmem_full[as]), (acc_bits >> as) & 1u, wc, kWaitTmemFull));
+                            if (!ok) break;
+                            acc_bits ^= 1u << as;
+                            tc_fence_after();
+                            const uint32_t taddr = lane_base + as * (kDecBlockQ * 16u * NUN);
+                            uint64_t a01 = 0ull, a23 = 0ull;
+                            uint32_t v[16];
+#pragma unroll
+                            for (uint32_t u = 0; u < 2u * NUN; ++u) {
+                                tmem_ld_x16(taddr + u * 16u, v);
+                                tmem_ld_wait();
+                                if (u + 1 == 2u * NUN) {
+                                    tc_fence_before();
+                                    if (lane == 0) mbar_arrive_n(smem_u32(&bars->tmem_empty[as]), kDecArrivals / 12u);
+                                }
+#pragma unroll
+                                for (uint32_t i = 0; i < 4; ++i) {
+                                    const float x0 = __uint_as_float(v[4 * i]), x1 = __uint_as_float(v[4 * i + 1]);
+                                    const float x2 = __uint_as_float(v[4 * i + 2]), x3 = __uint_as_float(v[4 * i + 3]);
+                                    a01 = fma_f32x2(pack_f32x2(relu_nan(x0), relu_nan(x1)), wp[8 * u + 2 * i], a01);
+                                    a23 = fma_f32x2(pack_f32x2(relu_nan(x2), relu_nan(x3)), wp[8 * u + 2 * i + 1], a23);
+                                }
+                                if ((u + 1) % NUN == 0) {
+                                    const bool second = u + 1 == 2u * NUN;
+                                    const uint32_t off = j - (second ? s1 : s0);
+                                    if (off < (second ? span1 : span0))
+                                        out[(second ? p.logits_stride : 0u) + off] = __float2bfloat16_rn((lo_f32(a01) + hi_f32(a01)) + (lo_f32(a23) + hi_f32(a23)));
+                                    a01 = a23 = 0ull;
+                                }
+                            }
+                        }
+                    } else {
+                        acc_bits ^= (((blocks + 1u) >> 1) & 1u) | (((blocks >> 1) & 1u) << 1);
+                    }
+                    continue;
+                }
                 if (DEC) {
                     // This warpgroup reduces query qi of every kv block with index = group (mod groups).  The ring of
                     // accumulator stages is walked over all kv blocks; a stage's barrier cannot be a use behind when it
                     // is waited on, because the ring has at least as many stages as there are groups, the commits
                     // complete in order, and no warp enters a task (w_full) before all have left the one before.
                     const uint32_t groups = 4u / k.nq, group = wg / k.nq, qi = wg - group * k.nq;
-                    const uint32_t width = k.nq * p.num_heads, stages = min(kDecStages, kDecAccCols / width);
+                    const uint32_t width = dec_width_q(k.nq) * 16u * NUN, stages = dec_stages(width);
                     const uint32_t blocks = k.kb1 - k.kb0, share = kDecArrivals / (4u * k.nq);
                     const uint32_t s_fix = win[qi], e_fix = win[16u + qi];
                     const uint32_t span = e_fix > s_fix ? e_fix - s_fix : 0u;

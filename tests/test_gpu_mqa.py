@@ -237,7 +237,7 @@ def test_mqa_logits_paged_many_requests(kind, H, page_kv):
                 assert err.item() <= 0.05
 
 
-@pytest.mark.parametrize("kind,H,page_kv", [("fp8", 64, 64), ("fp4", 64, 16)])
+@pytest.mark.parametrize("kind,H,page_kv", [("fp8", 64, 64), ("fp4", 64, 16), ("fp8", 32, 64), ("fp4", 32, 4)])
 def test_mqa_logits_paged_wide_requests(kind, H, page_kv):
     """Requests of three to fourteen tokens: several query blocks per request, full ones and remainders, every logit
     against the oracle."""
