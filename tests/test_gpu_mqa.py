@@ -271,3 +271,25 @@ def test_mqa_logits_paged_wide_requests(kind, H, page_kv):
         ref = o.mqa_logits_ref(qd[t], kvd[perm[r]].reshape(-1, D)[:c.max()], wb.float().numpy()[t], np.zeros(len(c), np.uint32), c)
         ref = np.pad(ref, ((0, 0), (0, width - ref.shape[1])))
         _check(got[t], o.bf16_bits_to_f32(o.f32_to_bf16_bits_np(ref)), np.zeros(len(c), np.uint32), c, width, fill)
+
+
+@pytest.mark.parametrize("T,S,sequences", [(3, 1100, 1), (64, 4100, 8), (130, 8200, 3)])
+@pytest.mark.parametrize("extra", [0, 8200])
+def test_mqa_logits_packed_windows(T, S, sequences, extra):
+    """Packed sequences, with logits rows as wide as the longest window and wider than the kv range: the number of
+    pieces a query block's kv range is cut into follows from that width, the logits do not."""
+    H, D = 64, 128
+    q8, kv8, scale, w = _inputs_f32(T, S, H, D, T)
+    win = []
+    for i in range(sequences):
+        q0, q1, k0, k1 = T * i // sequences, T * (i + 1) // sequences, S * i // sequences, S * (i + 1) // sequences
+        win += [(k0, k1 - (q1 - q0) + j + 1) for j in range(q1 - q0)]
+    ks, ke = np.array(win, dtype=np.uint32).T
+    width, fill = (int((ke - ks).max()) + 7) // 8 * 8 + extra, -7.0
+    logits = torch.full((T, width), fill, dtype=torch.float32, device="cuda")
+    mqa_logits_f32(dev(q8), dev(kv8), dev(scale), dev(w), dev(ks.view(np.int32)), dev(ke.view(np.int32)), T, S, H, D, logits, width)
+    poll_device_status()
+    got = logits.cpu().numpy()
+    rows = np.unique(np.concatenate([np.arange(0, T, 7), [T - 1]]))
+    ref = o.mqa_logits_ref(E4M3[q8[rows]], E4M3[kv8] * scale[:, None], w[rows], ks[rows], ke[rows])
+    _check(got[rows], ref, ks[rows], ke[rows], S, fill)
