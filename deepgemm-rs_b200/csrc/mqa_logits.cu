@@ -61,13 +61,12 @@ static_assert(mqa_launch_regs(8) == 168 && mqa_epilogue_regs(8) == 232, "registe
 constexpr uint32_t kDecStages = 6;         // decode: accumulator stages at most
 constexpr uint32_t kDecAccCols = 384;      // decode: columns they share
 constexpr uint32_t kDecArrivals = 48;      // decode: arrivals that free a stage, split evenly over its reducing warps (4, 8, 12 or 16)
-constexpr uint32_t kDecBlockQ = 6;         // decode: queries of a request per task
-// decode: queries the MMAs and the accumulator stages of a task are wide (nq rounded up: four widths, each with loops of its own)
-__host__ __device__ constexpr uint32_t dec_width_q(uint32_t nq) { return nq <= 2u ? nq : nq <= 4u ? 4u : 6u; }
+// decode, 16 * nun heads: queries of a request per task
+__host__ __device__ constexpr uint32_t dec_block_q(uint32_t nun) { return nun == 4u ? 3u : 6u; }
+// decode: queries the MMAs and the accumulator stages of a task are wide (nq rounded up to a few widths, each with an MMA loop of its own)
+__host__ __device__ constexpr uint32_t dec_width_q(uint32_t nun, uint32_t nq) { return nq <= 2u ? nq : nun == 4u ? 3u : nq <= 4u ? 4u : 6u; }
 __host__ __device__ constexpr uint32_t dec_stages(uint32_t width) { return kDecAccCols / width < kDecStages ? kDecAccCols / width : kDecStages; }
-// paged: block-table look-ups run so many kv blocks ahead (64 heads, 128 requests x 1 token over up to 8192: 30.4 us with
-// eight, 27.9 with four, the same over 32768; the decode form the other way round, 83.6 / 85.1 us over 32768)
-__host__ __device__ constexpr uint32_t pages_ahead(bool dec) { return dec ? 8u : 4u; }
+constexpr uint32_t kPagesAhead = 4;        // paged: block-table look-ups run so many kv blocks ahead
 constexpr uint32_t kMqaSfaCol = 448;       // ue8m0 contracts only: the accumulators are <= 192 wide
 constexpr uint32_t kMqaSfbCol = 452;
 
@@ -232,14 +231,13 @@ __device__ __forceinline__ float relu_nan(float x) {
 // U4: head counts that are not a multiple of 16 (their 4-column reduction loop is a variant of its own: as a
 // run-time branch beside the 16-column loop it cost the common case 4 %).
 // QPW: queries per warpgroup of the NUN variants (their NUN units are QPW queries of 16 * NUN / QPW heads).
-// DEC (paged, 32 heads): decode.  A request has one to four tokens, so with two queries per warpgroup most warpgroups
-// had nothing to reduce and the live ones ran at the latency of their TMEM loads.  Here the four
-// warpgroups take (query, kv block) pairs: with nq <= 4 queries in a task, 4 / nq kv blocks are reduced side by side, the
-// MMAs are only as wide as the queries need and the accumulator ring has as many stages as then fit in kDecAccCols
-// columns.  Five or six queries go to three warpgroups, two each (with four per task at most, requests of five and six
-// tokens read their cache twice: 64 requests x 6 tokens over up to 8192 took 33.2 us instead of 26.4).
-// (128 requests x 2 tokens over up to 32768: 103 -> 83 us.  64 heads are as fast without it for one or two tokens, 101.5 /
-// 101.3 us, and slower with it for three, 41.2 / 36.1 us over up to 8192: they keep one query per warpgroup.)
+// DEC (paged, 32 or 64 heads): decode.  A request has few tokens, so with a fixed share of the query block per warpgroup
+// most warpgroups had nothing to reduce and the live ones ran at the latency of their TMEM loads.  Here, up to two (64
+// heads) or four (32) queries in a task, the four warpgroups take (query, kv block) pairs: 4 / nq kv blocks are reduced
+// side by side, the MMAs are only as wide as the queries need and the accumulator ring has as many stages as then fit in
+// kDecAccCols columns.  Wider tasks go to three warpgroups, 64 columns each, over two stages.  Microseconds without / with
+// this form, over contexts of up to 8192 tokens, 128 requests of 1, 2, 3 tokens and 64 of 6: 64 heads 34.7 / 26.6,
+// 36.0 / 31.1, 42.8 / 40.3, 35.9 / 35.1; 32 heads 34.6 / 26.1, 34.9 / 28.0, 39.2 / 32.3, 26.7 / 25.0.
 // NUN: 16-column units a warpgroup reduces per kv block when that is known at compile time (4 / 8 = one query of
 // 64 / 128 heads per warpgroup: the unit loop is then straight-line code without counters), 0 = any.
 template <bool SCALED, bool FP4, bool PAGED, bool U4 = false, uint32_t NUN = 0, uint32_t QPW = 1, bool DEC = false>
@@ -258,7 +256,6 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const WaitCtx wc{p.status, &bars->abort};
     const uint32_t ep_warps = 4u * p.ep_groups;
-    constexpr uint32_t kAhead = pages_ahead(DEC);
 
     if (threadIdx.x == 0) {
         bars->abort = 0;
@@ -328,12 +325,12 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     const uint32_t pg = tok_of(kbx) >> page_shift;
                     return (kbx < k.kb1 && lane < p.boxes_per_block && pg < p.block_table_stride) ? __ldg(trow + pg) : 0u;
                 };
-                uint32_t pq[kAhead];
+                uint32_t pq[kPagesAhead];
 #pragma unroll
-                for (uint32_t j = 0; j < kAhead; ++j) pq[j] = page_of(k.kb0 + j);
-                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kAhead) {
+                for (uint32_t j = 0; j < kPagesAhead; ++j) pq[j] = page_of(k.kb0 + j);
+                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kPagesAhead) {
 #pragma unroll
-                    for (uint32_t j = 0; j < kAhead; ++j) {
+                    for (uint32_t j = 0; j < kPagesAhead; ++j) {
                         const uint32_t kb = kb0 + j;
                         if (kb >= k.kb1) break;
                         if (!(ok = DG_WARP_WAIT(smem_u32(&bars->kv_empty[stage]), phase ^ 1u, wc, kWaitEmpty))) break;
@@ -342,7 +339,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         // rows past the table's width or pages outside the cache read row 0 (paged_row)
                         uint32_t row = pq[j] * p.page_kv + (tok_of(kb) & (p.page_kv - 1u));
                         if (row + p.box_rows > p.num_kv) row = 0u;
-                        pq[j] = page_of(kb + kAhead);
+                        pq[j] = page_of(kb + kPagesAhead);
                         if (lane == 0) mbar_arrive_expect_tx(bar, kv_tx);
                         __syncwarp();
                         if (lane < p.boxes_per_block) tma_load_2d(&tm_kv, bar, dst + lane * p.box_rows * p.row_bytes, 0, (int32_t)row);
@@ -369,6 +366,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // ===================================================== MMA issuer (warp-converged, one lane issues)
         uint32_t stage = 0, phase = 0, qcount = 0, acount = 0;
         uint32_t acc_bits = 0;      // DEC: per accumulator stage, parity of its uses so far
+        uint32_t ring = 0, ring_q = 0;   // DEC: next accumulator stage, width of the ring in queries
         bool ok = true;
         MqaTasks<PAGED> tasks(p);
         MqaTask k;
@@ -397,14 +395,16 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             // at that pace (128 requests x 2 tokens over up to 32768: 82.6 us, with constants 72.8)
             auto kv_loop = [&](auto width_q) {
             constexpr uint32_t WQ = decltype(width_q)::value;
-            // DEC: width and number of the accumulator stages of this task; the ring starts over at its first stage once
-            // every stage of the task before (of another width, maybe) has been drained
+            // A task as wide as the one before goes on in its ring; for another width the ring starts over at its first stage once
+            // every stage of the old one has been drained.
             constexpr uint32_t kWidth = WQ * 16u * NUN, kStages = WQ ? dec_stages(kWidth ? kWidth : 1u) : 0u;
             const uint32_t idesc = DEC ? make_idesc_bs(FP4 ? 1u : 0u, FP4 ? 1u : 0u, kMqaBlockKv, kWidth) : p.idesc;
-            uint32_t ring = 0;
-            if (DEC)
+            if (DEC && ring_q != WQ) {
                 for (uint32_t s = 0; ok && s < kDecStages; ++s)
                     ok = wait_on(smem_u32(&bars->tmem_empty[s]), ((acc_bits >> s) & 1u) ^ 1u, kWaitTmemEmpty);
+                ring = 0;
+                ring_q = WQ;
+            }
             for (uint32_t kb = k.kb0; ok && kb < k.kb1; ++kb) {
                 if (!(ok = wait_on(smem_u32(&bars->kv_full[stage]), phase, kWaitFull))) break;
                 if (SCALED && !PAGED && !(ok = wait_on(smem_u32(&bars->kv_ready[stage]), phase, kWaitSfReady))) break;
@@ -454,8 +454,8 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             if constexpr (!DEC) kv_loop(std::integral_constant<uint32_t, 0>{});
             else if (k.nq == 1u) kv_loop(std::integral_constant<uint32_t, 1>{});
             else if (k.nq == 2u) kv_loop(std::integral_constant<uint32_t, 2>{});
-            else if (k.nq <= 4u) kv_loop(std::integral_constant<uint32_t, 4>{});
-            else kv_loop(std::integral_constant<uint32_t, 6>{});
+            else if (k.nq <= (NUN == 4u ? 3u : 4u)) kv_loop(std::integral_constant<uint32_t, dec_width_q(NUN, 3)>{});
+            else kv_loop(std::integral_constant<uint32_t, dec_width_q(NUN, 6)>{});
             }
             if (kLaneLoop) {
                 // the other lanes take over the issuer's position in the rings
@@ -464,6 +464,8 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 phase = __shfl_sync(0xffffffffu, phase, issuer_lane);
                 acount = __shfl_sync(0xffffffffu, acount, issuer_lane);
                 acc_bits = __shfl_sync(0xffffffffu, acc_bits, issuer_lane);
+                ring = __shfl_sync(0xffffffffu, ring, issuer_lane);
+                ring_q = __shfl_sync(0xffffffffu, ring_q, issuer_lane);
                 ok = __shfl_sync(0xffffffffu, (uint32_t)ok, issuer_lane) != 0u;
             }
         }
@@ -505,19 +507,19 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     const uint32_t pg = (kbx * kMqaBlockKv + 4u * lane) >> page_shift;
                     return (kbx < k.kb1 && pg < p.block_table_stride) ? __ldg(trow + pg) : 0u;
                 };
-                uint32_t pq[kAhead];
+                uint32_t pq[kPagesAhead];
 #pragma unroll
-                for (uint32_t j = 0; j < kAhead; ++j) pq[j] = page_of(k.kb0 + j);
-                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kAhead) {
+                for (uint32_t j = 0; j < kPagesAhead; ++j) pq[j] = page_of(k.kb0 + j);
+                for (uint32_t kb0 = k.kb0; ok && kb0 < k.kb1; kb0 += kPagesAhead) {
 #pragma unroll
-                    for (uint32_t j = 0; j < kAhead; ++j) {
+                    for (uint32_t j = 0; j < kPagesAhead; ++j) {
                         const uint32_t kb = kb0 + j;
                         if (kb >= k.kb1) break;
                         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->kv_empty[stage]), phase ^ 1u, wc, kWaitEmpty));
                         if (!ok) break;
                         uint32_t row = pq[j] * p.page_kv + ((kb * kMqaBlockKv + 4u * lane) & (p.page_kv - 1u));
                         if (row + 4u > p.num_kv) row = 0u;       // tokens past the table or the cache: masked by the epilogue
-                        pq[j] = page_of(kb + kAhead);
+                        pq[j] = page_of(kb + kPagesAhead);
                         // row r = 4 l + i of the block goes to position 4 (r % 32) + r / 32
                         const uint32_t sf = base + p.off_kv + stage * p.kv_stage_bytes + p.kv_sf_off + (lane >> 3) * 4u;
 #pragma unroll
@@ -548,7 +550,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         const uint32_t et = threadIdx.x - 128u;
         const uint32_t wg = et >> 7;                  // warpgroup index
         const uint32_t quarter = warp & 3u;           // TMEM lane quarter of this warp
-        uint32_t qcount = 0, acount = 0, acc_bits = 0;
+        uint32_t qcount = 0, acount = 0, acc_bits = 0, ring = 0, ring_q = 0;
         bool ok = true;
         MqaTasks<PAGED> tasks(p);
         MqaTask k;
@@ -600,40 +602,45 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 if (lane == 0) mbar_arrive(smem_u32(&bars->w_full[wb]));
                 ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->w_full[wb]), wphase, wc, kWaitWeights));
                 if (!ok) break;
-                if (DEC && k.nq > 4u) {
-                    // Two queries per warpgroup, three warpgroups, two accumulator stages in turn; the fourth warpgroup only
-                    // keeps count of their uses.
-                    constexpr uint32_t kStages = dec_stages(kDecBlockQ * 16u * (NUN ? NUN : 1u));
-                    static_assert(!DEC || kStages == 2u, "stages in turn");
+                if (DEC && ring_q != dec_width_q(NUN, k.nq)) {      // the ring starts over, as in the MMA issuer
+                    ring = 0;
+                    ring_q = dec_width_q(NUN, k.nq);
+                }
+                if (DEC && k.nq > (NUN == 4u ? 2u : 4u)) {
+                    // One query (64 heads) or two (32) per warpgroup, three warpgroups, two accumulator stages in turn; the
+                    // fourth warpgroup only keeps count of their uses.
+                    constexpr uint32_t kQ = dec_block_q(NUN) / 3u, kCols = dec_block_q(NUN) * 16u * (NUN ? NUN : 1u);
+                    static_assert(!DEC || (dec_stages(kCols) == 2u && kQ * NUN == 4u), "stages in turn, 64 columns per warpgroup");
                     const uint32_t blocks = k.kb1 - k.kb0;
                     if (wg < 3u) {
-                        const uint32_t qi = 2u * wg;
-                        const uint32_t s0 = win[qi], e0 = win[16u + qi], s1 = win[qi + 1u], e1 = win[17u + qi];   // e = 0: no such query
+                        const uint32_t qi = kQ * wg, last = qi + kQ - 1u;
+                        const uint32_t s0 = win[qi], e0 = win[16u + qi], s1 = win[last], e1 = win[16u + last];   // e = 0: no such query
                         const uint32_t span0 = e0 > s0 ? e0 - s0 : 0u, span1 = e1 > s1 ? e1 - s1 : 0u;
                         __nv_bfloat16* const out = reinterpret_cast<__nv_bfloat16*>(p.logits) + (size_t)(k.q0 + qi) * p.logits_stride;
                         const uint32_t lane_base = tmem + ((quarter * 32u) << 16) + qi * 16u * NUN;
-                        uint64_t wp[NUN ? 16u * NUN : 1u];
+                        uint64_t wp[32];
 #pragma unroll
-                        for (uint32_t i = 0; i < 8u * NUN; ++i) {
+                        for (uint32_t i = 0; i < 16u; ++i) {
                             const float4 w4 = reinterpret_cast<const float4*>(w + qi * 16u * NUN)[i];
                             wp[2 * i] = pack_f32x2(w4.x, w4.y);
                             wp[2 * i + 1] = pack_f32x2(w4.z, w4.w);
                         }
                         uint32_t j = k.kb0 * kMqaBlockKv + quarter * 32u + lane;
                         for (uint32_t b = 0; b < blocks; ++b, j += kMqaBlockKv) {
-                            const uint32_t as = b & 1u;
+                            const uint32_t as = ring;
                             ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->tmem_full[as]), (acc_bits >> as) & 1u, wc, kWaitTmemFull));
                             if (!ok) break;
                             acc_bits ^= 1u << as;
+                            ring ^= 1u;
                             tc_fence_after();
-                            const uint32_t taddr = lane_base + as * (kDecBlockQ * 16u * NUN);
+                            const uint32_t taddr = lane_base + as * kCols;
                             uint64_t a01 = 0ull, a23 = 0ull;
                             uint32_t v[16];
 #pragma unroll
-                            for (uint32_t u = 0; u < 2u * NUN; ++u) {
+                            for (uint32_t u = 0; u < 4u; ++u) {
                                 tmem_ld_x16(taddr + u * 16u, v);
                                 tmem_ld_wait();
-                                if (u + 1 == 2u * NUN) {
+                                if (u + 1 == 4u) {
                                     tc_fence_before();
                                     if (lane == 0) mbar_arrive_n(smem_u32(&bars->tmem_empty[as]), kDecArrivals / 12u);
                                 }
@@ -644,8 +651,8 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                                     a01 = fma_f32x2(pack_f32x2(relu_nan(x0), relu_nan(x1)), wp[8 * u + 2 * i], a01);
                                     a23 = fma_f32x2(pack_f32x2(relu_nan(x2), relu_nan(x3)), wp[8 * u + 2 * i + 1], a23);
                                 }
-                                if ((u + 1) % NUN == 0) {
-                                    const bool second = u + 1 == 2u * NUN;
+                                if ((u + 1) % (NUN ? NUN : 1u) == 0) {
+                                    const bool second = kQ == 2u && u + 1 == 4u;
                                     const uint32_t off = j - (second ? s1 : s0);
                                     if (off < (second ? span1 : span0))
                                         out[(second ? p.logits_stride : 0u) + off] = __float2bfloat16_rn((lo_f32(a01) + hi_f32(a01)) + (lo_f32(a23) + hi_f32(a23)));
@@ -654,7 +661,8 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                             }
                         }
                     } else {
-                        acc_bits ^= (((blocks + 1u) >> 1) & 1u) | (((blocks >> 1) & 1u) << 1);
+                        acc_bits ^= ((((blocks + 1u) >> 1) & 1u) << ring) | (((blocks >> 1) & 1u) << (ring ^ 1u));
+                        ring ^= blocks & 1u;
                     }
                     continue;
                 }
@@ -664,7 +672,7 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     // is waited on, because the ring has at least as many stages as there are groups, the commits
                     // complete in order, and no warp enters a task (w_full) before all have left the one before.
                     const uint32_t groups = 4u / k.nq, group = wg / k.nq, qi = wg - group * k.nq;
-                    const uint32_t width = dec_width_q(k.nq) * 16u * NUN, stages = dec_stages(width);
+                    const uint32_t width = ring_q * 16u * NUN, stages = dec_stages(width);
                     const uint32_t blocks = k.kb1 - k.kb0, share = kDecArrivals / (4u * k.nq);
                     const uint32_t s_fix = win[qi], e_fix = win[16u + qi];
                     const uint32_t span = e_fix > s_fix ? e_fix - s_fix : 0u;
@@ -677,12 +685,12 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         wp[2 * i] = pack_f32x2(w4.x, w4.y);
                         wp[2 * i + 1] = pack_f32x2(w4.z, w4.w);
                     }
-                    uint32_t as = 0, turn = 0;               // stage and (block index mod groups) of the current kv block
+                    uint32_t turn = 0;                       // block index mod groups
                     for (uint32_t b = 0; b < blocks; ++b) {
-                        const uint32_t aphase = (acc_bits >> as) & 1u, cur = as;
+                        const uint32_t aphase = (acc_bits >> ring) & 1u, cur = ring;
                         const bool mine = turn == group;
-                        acc_bits ^= 1u << as;
-                        if (++as == stages) as = 0;
+                        acc_bits ^= 1u << ring;
+                        if (++ring == stages) ring = 0;
                         if (++turn == groups) turn = 0;
                         if (!mine) continue;
                         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->tmem_full[cur]), aphase, wc, kWaitTmemFull));
@@ -737,21 +745,6 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         wp[2 * i + 1] = pack_f32x2(w4.z, w4.w);
                     }
                     uint32_t j = k.kb0 * kMqaBlockKv + quarter * 32u + lane;
-                    // A warpgroup none of whose queries the task has (decode: one or two tokens of a request in a block
-                    // of three) only hands the accumulator stages back; its issue slots go to the others.
-                    // (A loop of its own: as a branch inside the reduction loop below it cost that loop 17 %.)
-                    if (PAGED && q_first >= k.nq) {
-                        for (uint32_t kb = k.kb0; kb < k.kb1; ++kb) {
-                            const uint32_t as = acount & 1u, aphase = (acount >> 1) & 1u;
-                            ++acount;
-                            ok = __all_sync(0xffffffffu, mbar_wait(full0 + as * 8u, aphase, wc, kWaitTmemFull));
-                            if (!ok) break;
-                            tc_fence_after();
-                            tc_fence_before();
-                            if (lane == 0) mbar_arrive(empty0 + as * 8u);
-                        }
-                        continue;
-                    }
                     for (uint32_t kb = k.kb0; kb < k.kb1; ++kb, j += kMqaBlockKv) {
                         const uint32_t as = acount & 1u, aphase = (acount >> 1) & 1u;
                         ++acount;
@@ -1006,9 +999,9 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
     // columns of the ue8m0 contracts keep all three (six) queries that fit, on three warpgroups (one query of 64
     // heads or two of 32 each): with two queries the MMAs are 128 columns wide and only eight warps reduce.
     const bool three_groups = SCALED && ((num_heads == 64 && block_q == 3) || (num_heads == 32 && block_q == 6));
-    // decode: one to four tokens of a request, four warpgroups over (query, kv block) pairs
-    const bool dec = PAGED && num_heads == 32;
-    if (dec) block_q = kDecBlockQ;
+    // decode: few tokens of a request, four warpgroups over (query, kv block) pairs
+    const bool dec = PAGED && (num_heads == 64 || num_heads == 32);
+    if (dec) block_q = dec_block_q(num_heads / 16u);
     else if (three_groups) { /* keep */ }
     else if (block_q >= 4) block_q &= ~3u;
     else if (block_q == 3) block_q = 2;
@@ -1202,15 +1195,14 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
     };
     e = cudaSuccess;
     bool done = false;
-    if (num_heads == 64 && p.block_q == p.ep_groups) {
-        done = true;
-        run(mqa_logits_kernel<SCALED, FP4, PAGED, false, 4>, 4);                                          // one query of 64 heads per warpgroup
-    } else if constexpr (PAGED) {
+    if constexpr (PAGED) {
         done = dec;
-        if (dec) run(mqa_logits_kernel<SCALED, FP4, true, false, 2, 1, true>, 4);
+        if (dec && num_heads == 64) run(mqa_logits_kernel<SCALED, FP4, true, false, 4, 1, true>, 4);
+        else if (dec) run(mqa_logits_kernel<SCALED, FP4, true, false, 2, 1, true>, 4);
     } else {
-        done = num_heads == 32 && p.block_q == 2u * p.ep_groups && p.ep_groups >= 3u;
-        if (done) run(mqa_logits_kernel<SCALED, FP4, false, false, 4, 2>, 4);                             // two queries of 32 heads per warpgroup
+        done = (num_heads == 32 && p.block_q == 2u * p.ep_groups && p.ep_groups >= 3u) || (num_heads == 64 && p.block_q == p.ep_groups);
+        if (done && num_heads == 32) run(mqa_logits_kernel<SCALED, FP4, false, false, 4, 2>, 4);     // two queries of 32 heads per warpgroup
+        else if (done) run(mqa_logits_kernel<SCALED, FP4, false, false, 4>, 4);                      // one query of 64 heads per warpgroup
     }
     if (!done) {
         if (p.unit == 4u) run(mqa_logits_kernel<SCALED, FP4, PAGED, true>, 0);
