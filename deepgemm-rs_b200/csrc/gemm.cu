@@ -1104,6 +1104,18 @@ static void pick_scaled_tile(const TileTimes& times, uint32_t m, uint32_t groups
     }
 }
 
+// BF16 GEMMs with an MN-major operand: CTA pairs or single CTAs.  A pair needs a tile of 128 columns at least where a
+// single CTA has 64, starts about 0.8 us later and then saves a tenth or more per k-block when there are tiles enough.  Device
+// times, pairs / single CTAs, over 483 shapes (129 to 4096 x 512 to 7168, K 256 to 7168), tiles = 128 x 64 blocks of D: nn with
+// tiles <= 148 1.18 (K 256) to 1.02 (K 7168); tiles 149 to 600 1.15, 1.10, 1.04, 1.01, 0.97, 0.92 (K 256, 512, 1024, ... 7168);
+// 601 to 1100 1.03, then 0.97 to 0.88; beyond 0.94 to 0.81; tt alike.  With a K-major B (tn) the loads gain nothing:
+// 0.99 on the average where there are more than 300 tiles and K is 4096 or more, 0.90 at best, and above 1 elsewhere.
+static bool mn_major_on_pairs(uint32_t m, uint32_t n, uint32_t k, bool b_mn, uint32_t sms) {
+    const uint64_t tiles = (uint64_t)ceil_div(m, kBlockM) * ceil_div(n, 64u);
+    if (!b_mn) return tiles > 2u * sms && k >= 4096u;
+    return tiles > 8u * sms || (tiles > 4u * sms && k >= 512u) || (tiles > sms && k >= 2048u);
+}
+
 static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k, uint32_t num_groups,
                          uint32_t expected_m, uint32_t gran_a, uint32_t gran_b, const DeviceInfo* dev, Plan* plan,
                          bool allow_dynamic = true, bool a_mn = false, bool b_mn = false, bool plain = true) {
@@ -1132,9 +1144,9 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     const uint32_t forced_cl = env_u32("DG_CLUSTER", 0);
     if (forced_cl == 1 || forced_cl == 2) cl = forced_cl;
     if (gtype == kContiguous && m / kBlockM > kMaxPairedBlocks) cl = 1;   // the in-kernel tile list is bounded
-    // MN-major tiles: BF16 GEMMs run on pairs as well (every CTA loads whole swizzle atoms of its share); FP8 atoms are
+    // MN-major tiles: large BF16 GEMMs run on pairs as well (every CTA loads whole swizzle atoms of its share); FP8 atoms are
     // 128 columns, and two of them per CTA would be wider than the accumulators beside the scale factors.
-    if ((a_mn || b_mn) && (kind != kBf16 || gtype != kNormal)) cl = 1;
+    if ((a_mn || b_mn) && (kind != kBf16 || gtype != kNormal || (forced_cl == 0 && !mn_major_on_pairs(m, n, k, b_mn, sms)))) cl = 1;
     uint32_t dense_bn = 0;
     const TileTimes& times = kind == kFp4 ? kFp4Times : (gran_a == 128 && gran_b == 128) ? kFp8Per128 : kFp8Per32;
     if (kind != kBf16 && gtype != kContiguous && !a_mn && !b_mn && (gtype == kMasked || m > kBlockM) && forced_cl == 0 &&

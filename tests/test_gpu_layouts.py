@@ -202,10 +202,11 @@ def test_contiguous_gemm_recorded_into_a_cuda_graph():
 
 @pytest.mark.parametrize("layout", ["nn", "tn", "tt"])
 @pytest.mark.parametrize("m,n,k,f32", [(129, 64, 64, False), (257, 1048, 320, False), (640, 264, 2048, True), (512, 2048, 192, True)])
-def test_bf16_mn_major_views_on_cta_pairs(layout, m, n, k, f32):
-    """BF16 with more than one 128-row block runs on CTA pairs: second CTAs without rows or columns, a second half of B
-    outside the tensor, and accumulation into f32."""
+def test_bf16_mn_major_views_on_cta_pairs(layout, m, n, k, f32, monkeypatch):
+    """BF16 on CTA pairs: second CTAs without rows or columns, a second half of B outside the tensor, and accumulation
+    into f32 (forced: by itself the library puts problems of this size on single CTAs)."""
     from helpers import bf16_operand
+    monkeypatch.setenv("DG_CLUSTER", "2")
     a, fa = bf16_operand(randn((m, k), m))
     b, fb = bf16_operand(randn((n, k), n + 1))
     out = new_output(m, n, f32=f32, fill=1.5 if f32 else None)
@@ -218,3 +219,29 @@ def test_bf16_mn_major_views_on_cta_pairs(layout, m, n, k, f32):
     poll_device_status()
     ref = o.gemm_f32_ref(fa, fb)
     assert_close_to_oracle(to_f32(out), ref + 1.5 if f32 else bf16_round(ref), "bf16", f"{layout} {m}x{n}x{k}")
+
+
+@pytest.mark.parametrize("layout,m,n,k,cluster", [
+    ("nn", 256, 1024, 7168, 1),       # one wave of 64-wide single tiles: never pairs
+    ("nn", 1024, 2048, 1984, 1), ("nn", 1024, 2048, 2048, 2),
+    ("tt", 2048, 3072, 448, 1), ("tt", 2048, 3072, 512, 2), ("tt", 4096, 3072, 64, 2),
+    ("tn", 1024, 4096, 4032, 1), ("tn", 1024, 4096, 4096, 2), ("tn", 129, 512, 7168, 1),
+])
+def test_bf16_mn_major_choice_of_pairs(layout, m, n, k, cluster, monkeypatch, capfd):
+    """Both sides of every line of the rule, against float32 on the GPU: f32 outputs of sums of k products (2^-24 per
+    addition at most, random signs)."""
+    monkeypatch.setenv("DG_PRINT_CONFIGS", "1")
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    x, w = (torch.randn(r, k, device="cuda", generator=g).to(torch.bfloat16) for r in (m, n))
+    a, b = Operand.k_major(Dtype.Bf16, m, k, k, None, x), Operand.k_major(Dtype.Bf16, n, k, k, None, w)
+    out = new_output(m, n, f32=True)
+    if layout == "nn":
+        gemm_nn(a, mn_view(b), out)
+    elif layout == "tn":
+        gemm_tn(mn_view(a), b, out)
+    else:
+        gemm_tt(mn_view(a), mn_view(b), out)
+    poll_device_status()
+    assert f"cluster={cluster} " in capfd.readouterr().err
+    ref = x.double() @ w.double().t()
+    assert (out.data.double() - ref).abs().max().item() <= k * 2.0 ** -24 * k ** 0.5 + 1e-4
