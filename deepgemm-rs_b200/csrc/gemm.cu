@@ -625,7 +625,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     if (!SFW) {
                         if (lane == 0) {
                             if (CL == 1 || leader) mbar_arrive(smem_u32(&bars->sf_ready[stage]));
-                            else mbar_arrive_cluster(mapa(smem_u32(&bars->sf_ready[stage]), 0));
+                            else mbar_arrive_remote_own_data(mapa(smem_u32(&bars->sf_ready[stage]), 0));
                         }
                     } else {
                         const uint32_t set = n_sf & 1u;
@@ -793,7 +793,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                         __syncwarp();
                         if (lane == 0) {
                             if (CL == 1 || leader) mbar_arrive(smem_u32(&bars->tmem_empty[as]));
-                            else mbar_arrive_cluster(mapa(smem_u32(&bars->tmem_empty[as]), 0));
+                            else mbar_arrive_remote_own_data(mapa(smem_u32(&bars->tmem_empty[as]), 0));
                         }
                     }
                     if (col0 >= n_end) continue;
@@ -938,7 +938,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     __syncwarp();
                     if (lane == 0) {
                         if (CL == 1 || leader) mbar_arrive(smem_u32(&bars->tmem_empty[as]));
-                        else mbar_arrive_cluster(mapa(smem_u32(&bars->tmem_empty[as]), 0));
+                        else mbar_arrive_remote_own_data(mapa(smem_u32(&bars->tmem_empty[as]), 0));
                     }
                 }
                 const uint32_t col0 = t.n0 + c * 32u;

@@ -83,10 +83,15 @@ __device__ __forceinline__ uint32_t mapa(uint32_t local_addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
     return r;
 }
-// The release is at the instruction's default scope: as .release.cluster this arrive held its warp for 1500 to 1640
-// cycles on B200 (the partner's scale-factor warp then set the pace of a CTA pair).  What it publishes is read in the
-// CTA that arrives -- its own shared memory, which its own tensor core reads behind a proxy fence, and its own TMEM.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+// Arrival on another CTA's barrier.  `cluster_addr`: shared::cluster address of the barrier.
+// The plain form releases at the instruction's default scope, .cta: it orders nothing towards the other CTA's threads, so
+// it must not publish data that they read.  Its callers hand over what their own CTA's tensor core uses next on behalf
+// of the pair -- scale-factor words in this CTA's shared memory, an accumulator stage in this CTA's tensor memory -- and
+// each has completed its accesses first: every writing lane by fence.proxy.async and a warp barrier (the words are in
+// shared memory, ready for the asynchronous proxy), every reading lane by tcgen05.wait::ld and
+// tcgen05.fence::before_thread_sync (the columns are in registers).  As .release.cluster the arrival held its warp for
+// 1500 to 1640 cycles on B200, and the partner's scale-factor warp then set the pace of a CTA pair.
+__device__ __forceinline__ void mbar_arrive_remote_own_data(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 

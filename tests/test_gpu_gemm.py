@@ -462,3 +462,22 @@ def test_m_grouped_contiguous_choice_of_pairs(groups, n, k, blocks):
 def test_scale_factors_on_every_k_block_on_pairs(kind, gran, m, n, k):
     """FP8 per-32 and FP4 with more than one row block run on CTA pairs: ragged rows, a second CTA with one row, narrow tiles."""
     run_dense(kind, m, n, k, gran_a=gran, gran_b=gran, seed=m + n)
+
+
+@pytest.mark.parametrize("kind,gran", [("fp8", 128), ("fp8", 32), ("fp4", 32)])
+def test_pairs_equal_single_ctas_over_many_k_blocks(kind, gran):
+    """Scale factors of a pair cross from the partner's shared memory into tensor memory on the leader's word, and
+    accumulator stages come back: several tiles per pair, 128 (FP4: 64) k-blocks each, twenty launches in a row, all
+    the same bit for bit as on single CTAs."""
+    m, n, k = 3072, 4096, 16384
+    a, _ = quantised_operand(randn((m, k), 71), kind, gran)
+    b, _ = quantised_operand(randn((n, k), 72), kind, gran)
+    outs = []
+    for cluster, launches in (("1", 1), ("2", 20)):
+        os.environ["DG_CLUSTER"] = cluster
+        os.environ["DG_BLOCK_N"] = "208" if cluster == "1" else "224"
+        for _ in range(launches):
+            outs.append(new_output(m, n))
+            gemm_nt(a, b, outs[-1])
+    poll_device_status()
+    assert all(torch.equal(outs[0].data, x.data) for x in outs[1:])
