@@ -114,17 +114,22 @@ struct Tile {
 // A tile is (128 * CL) x BLOCK_N; CTA `rank` of a pair owns rows [rank*128, rank*128 + 128) of it.
 // Tile ids walk bands of `band` m-tiles, m fastest inside a band, so that the tiles in flight
 // share a few A row-blocks and B column-blocks in L2.
-// DYN (contiguous layout, single CTA): tile ids are not strided but claimed one by one from a global
+// DYN (contiguous layout): tile ids are not strided but claimed one by one from a global
 // counter by the CTA's scheduler warp and handed to the roles through a small ring in shared memory,
 // so that a CTA that is slowed down (an SM shared with another kernel, a slow tile) simply takes
-// fewer tiles instead of holding up the whole grid.
+// fewer tiles instead of holding up the whole grid.  On CTA pairs the leader's scheduler warp claims for both CTAs and
+// sends the id to the partner's ring as well; the partner's scheduler warp hands a slot back once its roles have read it.
+// Beside a kernel that keeps 8 SMs for milliseconds at a time, N 4096, K 7168: 64 experts of 384 rows 1197 us with strided
+// pair tiles, 839 claimed (single CTAs claimed 841); 16 experts of 1024 rows 626 and 448 (526).  Alone the two forms are
+// within 1 % there, at K 2048 (tiles of 6 us) claiming costs 2 %.
 constexpr uint32_t kSchedRing = 4;
+__host__ __device__ constexpr uint32_t sched_ring(int cl) { return cl == 2 ? 2u : kSchedRing; }   // slots in use: a pair's tiles are twice as large
 constexpr uint32_t kSchedRunBytes = 4096; // dynamic schedule: room for the run list behind the barrier block
 constexpr uint32_t kSchedMaxRuns = kSchedRunBytes / 2 - 1;   // runs of equal m_indices entries the scheduler warp keeps (u16 first blocks + end)
 struct SchedRing {
     uint64_t full[kSchedRing];     // scheduler warp -> roles: tile published
     uint64_t empty[kSchedRing];    // roles -> scheduler warp: every role has read the tile
-    uint64_t tile[kSchedRing];     // (m block << 32) | n block; m block 0xffffffff = no more tiles
+    uint64_t tile[kSchedRing];     // (m block << 32) | n block, on pairs the tile id; all ones = no more tiles
 };
 
 template <int GTYPE, int CL, bool SPLIT = false, bool DYN = false>
@@ -148,15 +153,19 @@ struct Scheduler {
         constexpr uint32_t kTileM = kBlockM * CL;
         uint32_t id = next_id;
         next_id += stride;
+        uint64_t ring_entry = 0;
         if (DYN) {
-            // the scheduler warp has already turned the claimed id into a tile (contiguous layout, one CTA)
+            // single CTAs: the scheduler warp has already turned the claimed id into a tile
             if (!DG_WARP_WAIT(smem_u32(&ring->full[slot]), ring_phase, *wc, kWaitSched)) return false;
-            const uint64_t entry = *reinterpret_cast<volatile uint64_t*>(&ring->tile[slot]);
+            ring_entry = *reinterpret_cast<volatile uint64_t*>(&ring->tile[slot]);
+            if (ring_entry == ~0ull) return false;      // the end is not handed back: nothing follows it in its slot
             __syncwarp();
             if ((threadIdx.x & 31u) == 0) mbar_arrive(smem_u32(&ring->empty[slot]));
-            if (++slot == kSchedRing) { slot = 0; ring_phase ^= 1u; }
-            const uint32_t mb = (uint32_t)(entry >> 32), nb = (uint32_t)entry;
-            if (mb == 0xffffffffu) return false;
+            if (++slot == sched_ring(CL)) { slot = 0; ring_phase ^= 1u; }
+            id = (uint32_t)ring_entry;
+        }
+        if (DYN && CL == 1) {
+            const uint32_t mb = (uint32_t)(ring_entry >> 32), nb = id;
             t.kb0 = 0; t.kb1 = p.num_k_blocks; t.split = 0;
             t.a_row = mb * kBlockM;
             t.row_end = p.m;
@@ -305,8 +314,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     // [tile list, 16 KB] only for the contiguous layout on CTA pairs
     uint16_t* mtiles = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(bars) + 1024);
     uint16_t* run_first = mtiles + kMaxPairedBlocks;    // [kMaxPairedBlocks + 1], padded to 17 KB
-    // [run list, 4 KB] only for the dynamic schedule
-    const uint32_t stages_base = smem_base + 1024u + (kPairedContig ? kPairedListBytes : 0u) + (DYN ? kSchedRunBytes : 0u);
+    // [run list, 4 KB] only for the dynamic schedule on single CTAs
+    const uint32_t stages_base = smem_base + 1024u + (kPairedContig ? kPairedListBytes : 0u) + (DYN && CL == 1 ? kSchedRunBytes : 0u);
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t rank = CL == 2 ? cluster_ctarank() : 0u;
@@ -327,10 +336,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             mbar_init(smem_u32(&bars->tmem_empty[s]), 4 * CL);
         }
         if (DYN) {
-            // readers of a tile id: producer, MMA issuer, (SF transposer,) four epilogue warps
+            // readers of a tile id: producer, MMA issuer, (SF transposer,) four epilogue warps; the leader of a pair counts the
+            // partner as one more, the partner has no MMA issuer
+            constexpr uint32_t kReaders = (kHasSf ? 7u : 6u) + (GA ? kGatherWarps : 0u);
             for (uint32_t s = 0; s < kSchedRing; ++s) {
                 mbar_init(smem_u32(&bars->sched.full[s]), 1);
-                mbar_init(smem_u32(&bars->sched.empty[s]), (kHasSf ? 7 : 6) + (GA ? kGatherWarps : 0u));
+                mbar_init(smem_u32(&bars->sched.empty[s]), CL == 1 ? kReaders : leader ? kReaders + 1u : kReaders - 1u);
             }
         }
         fence_barrier_init();
@@ -642,6 +653,45 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 if (++stage == p.num_stages) stage = 0;
             }
         }
+    } else if (DYN && CL == 2 && warp == 3 && leader) {
+        // ===================================================== tile scheduler of a pair (dynamic schedule)
+        const uint32_t total = n_mtiles * p.num_n_blocks;
+        uint32_t slot = 0, phase = 0;
+        bool first = true;      // the first tile of a pair is its own index: claimed like the others, a pair could take two of a few
+        for (;;) {
+            if (!DG_WARP_WAIT(smem_u32(&bars->sched.empty[slot]), phase ^ 1u, wc, kWaitSched)) break;
+            uint32_t id = 0;
+            if (lane == 0) {
+                id = first ? blockIdx.x / 2u : gridDim.x / 2u + atomicAdd(p.tile_counter, 1u);
+                first = false;
+                const uint64_t entry = id < total ? (uint64_t)id : ~0ull;
+                const uint32_t tile = smem_u32(&bars->sched.tile[slot]), full = smem_u32(&bars->sched.full[slot]);
+                st_async_b64(mapa(tile, 1), entry, mapa(full, 1));
+                *reinterpret_cast<volatile uint64_t*>(&bars->sched.tile[slot]) = entry;
+                mbar_arrive(full);
+            }
+            id = __shfl_sync(0xffffffffu, id, 0);
+            if (id >= total) break;                               // the roles read the end marker and stop as well
+            if (++slot == sched_ring(2)) { slot = 0; phase ^= 1u; }
+        }
+    } else if (DYN && CL == 2 && warp == 3) {
+        // ===================================================== the partner's end of it
+        // Every use of a slot is announced (eight bytes) before the leader is told that the slot is free.  The arrival
+        // over there is the slow one of cluster scope: it orders the roles' reads before the leader's next store.
+        uint32_t slot = 0, phase = 0;
+        if (lane == 0)
+            for (uint32_t s = 0; s < sched_ring(2); ++s) mbar_arrive_expect_tx(smem_u32(&bars->sched.full[s]), 8u);
+        for (;;) {
+            if (!DG_WARP_WAIT(smem_u32(&bars->sched.full[slot]), phase, wc, kWaitSched)) break;
+            if (*reinterpret_cast<volatile uint64_t*>(&bars->sched.tile[slot]) == ~0ull) break;
+            if (!DG_WARP_WAIT(smem_u32(&bars->sched.empty[slot]), phase, wc, kWaitSched)) break;
+            if (lane == 0) {
+                mbar_arrive_expect_tx(smem_u32(&bars->sched.full[slot]), 8u);
+                mbar_arrive_remote(mapa(smem_u32(&bars->sched.empty[slot]), 0));
+            }
+            __syncwarp();
+            if (++slot == sched_ring(2)) { slot = 0; phase ^= 1u; }
+        }
     } else if (DYN && warp == 3) {
         // ===================================================== tile scheduler (dynamic schedule)
         const uint32_t m_blocks = p.m_blocks_dev ? min(p.num_m_blocks, (uint32_t)__ldg(p.m_blocks_dev)) : p.num_m_blocks;
@@ -684,7 +734,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             uint32_t id = 0;
             if (lane == 0) id = atomicAdd(p.tile_counter, 1u);
             id = __shfl_sync(0xffffffffu, id, 0);
-            uint32_t mb = 0xffffffffu, nb = 0;
+            uint32_t mb = 0xffffffffu, nb = 0xffffffffu;
             if (id < total) {
                 uint32_t b0 = 0, b1 = m_blocks;                   // the run (or the whole layout) the tile lies in
                 if (n_runs) {
@@ -1029,7 +1079,7 @@ struct Plan {
     uint32_t grid;
     uint32_t num_tiles;
     uint32_t cluster;   // CTAs per tile: 1, or 2 (CTA pair)
-    bool dynamic;       // tiles claimed from a global counter instead of strided (contiguous layout, single CTA)
+    bool dynamic;       // tiles claimed from a global counter instead of strided (contiguous layout)
 };
 
 // A pair of zeroed counters for one launch of the dynamic schedule.  Launches take the pairs of the
@@ -1237,10 +1287,10 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     p.tx_sfa = sfa_bytes;
     p.tx_sfb = sfb_bytes;
     const uint32_t budget = (uint32_t)dev->smem_optin;
-    plan->dynamic = allow_dynamic && gtype == kContiguous && cl == 1 && p.k_splits == 1 && env_u32("DG_DYNAMIC", 1) != 0;
+    plan->dynamic = allow_dynamic && gtype == kContiguous && (cl == 1 || kind == kFp8) && p.k_splits == 1 && env_u32("DG_DYNAMIC", 1) != 0;
     const uint32_t fixed = 1024u /*alignment slack*/ + 1024u /*barriers*/ +
                            ((gtype == kContiguous && cl == 2) ? kPairedListBytes : 0u) /*tile and run lists*/ +
-                           (plan->dynamic ? kSchedRunBytes : 0u) /*run list of the scheduler warp*/;
+                           (plan->dynamic && cl == 1 ? kSchedRunBytes : 0u) /*run list of the scheduler warp*/;
     uint32_t stages = (budget - fixed) / p.stage_bytes;
     if (stages > kMaxStages) stages = kMaxStages;
     const uint32_t forced = env_u32("DG_NUM_STAGES", 0);
@@ -1558,6 +1608,7 @@ static int32_t run_gemm(const dg_operand_t* a, const dg_operand_t* b, dg_output_
     }
     if (plan.dynamic) {
         p.tile_counter = tile_counters(dev);
+        if (plan.cluster == 2) return launch<kFp8, kContiguous, 2, false, true>(plan, ta, tb, tsa, tsb, s);
         if (kind == kFp8 && sfw) return launch<kFp8, kContiguous, 1, false, true, false, true>(plan, ta, tb, tsa, tsb, s);
         if (kind == kFp8) return launch<kFp8, kContiguous, 1, false, true>(plan, ta, tb, tsa, tsb, s);
         if (kind == kFp4) return launch<kFp4, kContiguous, 1, false, true>(plan, ta, tb, tsa, tsb, s);

@@ -94,6 +94,16 @@ __device__ __forceinline__ uint32_t mapa(uint32_t local_addr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_remote_own_data(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// The form for everything else: what this thread has read or written before is ordered before what the other CTA's
+// threads do after their wait.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Eight bytes into another CTA's shared memory, counted by a barrier of that CTA (both shared::cluster addresses).
+__device__ __forceinline__ void st_async_b64(uint32_t cluster_dst, uint64_t v, uint32_t cluster_bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
+                 ::"r"(cluster_dst), "l"(v), "r"(cluster_bar) : "memory");
+}
 
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {

@@ -262,6 +262,7 @@ def test_m_grouped_contiguous(kind, cluster):
 def test_m_grouped_contiguous_many_blocks_random_runs():
     """A long random m_indices (runs of 1..5 blocks, padding blocks in between) on CTA pairs:
     exercises the in-kernel tile list over several 32-block chunks."""
+    os.environ["DG_CLUSTER"] = "2"
     rng = np.random.default_rng(5)
     groups, n, k = 8, 128, 256
     blocks = []
@@ -481,3 +482,27 @@ def test_pairs_equal_single_ctas_over_many_k_blocks(kind, gran):
             gemm_nt(a, b, outs[-1])
     poll_device_status()
     assert all(torch.equal(outs[0].data, x.data) for x in outs[1:])
+
+
+@pytest.mark.parametrize("groups,n,k,blocks", [
+    (2, 224, 512, [0, 0, 0, 1, 1]), (1, 1000, 1024, [0, 0, 0, -1, 0, 0, -1, 0, 0]),
+    (3, 4096, 512, [0] * 9 + [1] * 8 + [2] * 13),            # several tiles per pair
+    (1, 4096, 256, [-1] * 8),                                # no block in use
+])
+def test_m_grouped_contiguous_claimed_tiles_on_pairs(groups, n, k, blocks, monkeypatch):
+    """CTA pairs whose leader claims tiles for both CTAs: the result of strided tiles and of single CTAs bit for bit,
+    launch after launch (the counters are left at zero), with fewer tiles than pairs and with many per pair."""
+    m = 128 * len(blocks)
+    a, _ = quantised_operand(randn((m, k), 23), "fp8", 128)
+    b, _ = _stacked_b("fp8", groups, n, k, 24, gran=128)
+    indices = dev(np.array(blocks, dtype=np.int32))
+    got = []
+    for cluster, dynamic, launches in (("1", "0", 1), ("2", "0", 1), ("2", "1", 10)):
+        monkeypatch.setenv("DG_CLUSTER", cluster)
+        monkeypatch.setenv("DG_DYNAMIC", dynamic)
+        for _ in range(launches):
+            out = new_output(m, n, fill=3.0)
+            m_grouped_gemm_nt_contiguous(a, b, out, indices, groups)
+            got.append(out.data)
+    poll_device_status()
+    assert all(torch.equal(got[0], g) for g in got[1:])
