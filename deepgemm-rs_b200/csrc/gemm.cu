@@ -1138,8 +1138,9 @@ static const uint32_t kTileWidths[8] = {64, 96, 128, 160, 176, 192, 208, 224};
 static const TileTimes kFp8Per128 = {{181, 200, 248, 302, 331, 328, 369, 429}, {194, 210, 233, 277, 0, 302, 336, 367}};
 static const TileTimes kFp8Per32 = {{231, 228, 254, 322, 0, 344, 376, 441}, {0, 268, 279, 322, 0, 332, 363, 384}};    // either operand per 32
 static const TileTimes kFp4Times = {{214, 231, 254, 324, 0, 320, 354, 392}, {0, 303, 305, 363, 0, 364, 378, 385}};
-static void pick_scaled_tile(const TileTimes& times, uint32_t m, uint32_t groups, uint32_t n, uint32_t kb, uint32_t sms, uint32_t* cl_out,
-                             uint32_t* bn_out, bool pairs_allowed = true) {
+static double scaled_tile_ns(uint32_t cl, uint32_t kb, double per_kb) { return (cl == 1 ? 1300.0 : 400.0) + kb * per_kb; }
+static double pick_scaled_tile(const TileTimes& times, uint32_t m, uint32_t groups, uint32_t n, uint32_t kb, uint32_t sms, uint32_t* cl_out,
+                               uint32_t* bn_out, bool pairs_allowed = true) {
     double best = 1e30;
     for (uint32_t cl = 1; cl <= ((m > kBlockM && pairs_allowed) ? 2u : 1u); ++cl) {
         for (uint32_t i = 0; i < 8; ++i) {
@@ -1148,10 +1149,11 @@ static void pick_scaled_tile(const TileTimes& times, uint32_t m, uint32_t groups
             if (per_kb == 0) continue;
             const uint64_t tiles = (uint64_t)groups * ceil_div(m, kBlockM * cl) * ceil_div(n, bn);
             const uint64_t waves = (tiles + sms / cl - 1) / (sms / cl);
-            const double cost = (double)waves * ((cl == 1 ? 1300.0 : 400.0) + kb * per_kb);
+            const double cost = (double)waves * scaled_tile_ns(cl, kb, per_kb);
             if (cost < best) { best = cost; *cl_out = cl; *bn_out = bn; }
         }
     }
+    return best;
 }
 
 // BF16 GEMMs with an MN-major operand: CTA pairs or single CTAs.  A pair needs a tile of 128 columns at least where a
@@ -1178,19 +1180,10 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     p.num_k_blocks = k / block_k;
     // CTA pairs (256-row tiles) halve the B traffic per SM; they need at least two row blocks
     // that share B.  In the contiguous grouped layout the kernel pairs neighbouring blocks of one
-    // expert and runs an odd last block with an idle partner.
+    // expert and runs an odd last block with an idle partner (see below).
     const uint32_t rows_per_group = gtype == kMasked ? (expected_m ? expected_m : m) : m;
-    // Dense, masked and batched block-scaled GEMMs choose below, from measured tile times.  In the contiguous layout (FP8) an
-    // expert with an odd number of row blocks leaves half a pair idle, which costs time and energy.  Measured under
-    // lasting load, single CTAs / pairs (m counts the padding): 64 experts of 252 rows (m 24320) a whole feed-forward layer 1210 /
-    // 1165 us, 512 rows (m 40960) the GEMM 1105 / 1040 us, 32 experts of 1024 rows 968 / 884 us; but 256 experts of 512 rows
-    // (m 163584) a whole step 4990 / 5340 us.  So pairs are for layouts of about two and a half blocks per expert or more,
-    // beyond 65536 rows of eight blocks or more.  Layouts sized for the worst case (a device-side block count, rows stored
-    // through addresses) say nothing about their rows and share their SMs with transfers: single CTAs and the
-    // dynamic schedule.
-    const bool pair_contiguous = gtype == kContiguous && kind == kFp8 && gran_a == 128 && gran_b == 128 && plain && n >= 224u &&
-                                 (uint64_t)m >= (m <= 65536u ? 320ull : 1088ull) * num_groups;
-    uint32_t cl = (gtype == kContiguous ? pair_contiguous : rows_per_group > kBlockM) ? 2u : 1u;
+    // (block-scaled GEMMs choose below, from measured tile times)
+    uint32_t cl = gtype != kContiguous && rows_per_group > kBlockM ? 2u : 1u;
     const uint32_t forced_cl = env_u32("DG_CLUSTER", 0);
     if (forced_cl == 1 || forced_cl == 2) cl = forced_cl;
     if (gtype == kContiguous && m / kBlockM > kMaxPairedBlocks) cl = 1;   // the in-kernel tile list is bounded
@@ -1204,9 +1197,23 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
         pick_scaled_tile(times, rows_per_group, gtype == kNormal ? 1u : num_groups, n, p.num_k_blocks, sms, &cl, &dense_bn);   // masked: expected rows per group
     // the contiguous grouped layout on single CTAs: the same table (208 columns and five stages for N = 4096: 1994
     // against 1849 TFLOPS on 224 columns and four)
-    if (kind == kFp8 && gtype == kContiguous && cl == 1 && gran_a == 128 && gran_b == 128 && !a_mn && !b_mn && env_u32("DG_BLOCK_N", 0) == 0)
-        pick_scaled_tile(times, m, 1u, n, p.num_k_blocks, sms, &cl, &dense_bn, false);
-    if (pair_contiguous && cl == 2 && env_u32("DG_BLOCK_N", 0) == 0) dense_bn = 224u;   // the widest tile reads the least
+    if (kind == kFp8 && gtype == kContiguous && cl == 1 && gran_a == 128 && gran_b == 128 && !a_mn && !b_mn && env_u32("DG_BLOCK_N", 0) == 0) {
+        const double single_ns = pick_scaled_tile(times, m, 1u, n, p.num_k_blocks, sms, &cl, &dense_bn, false);
+        // Pairs, 224 columns (the widest tile reads the least): an expert with an odd number of row blocks leaves the second
+        // CTA of its last pair without work.  Time on pairs / on single CTAs under lasting load, both with claimed tiles, 40 layouts of
+        // 16 to 256 experts with 64 to 2048 rows (N, K 4096, 7168 and 7168, 2048), by the share of row blocks without a
+        // partner: 0.84 to 0.93 at up to 0.07, 0.88 to 0.97 at 0.1 to 0.16, 0.98 to 1.0 at 0.17 to 0.19, 1.04 to 1.07 at 0.33 to
+        // 0.37, 1.3 at 1.  The host does not know the layout, only its size: with six blocks per expert, padding included, five
+        // are in use and the share is a fifth at most whatever the routing.  (Smaller layouts gain or lose by the parity of
+        // their block counts: 64 experts of 252 rows 0.97, of 320 rows 1.05.)  The layout also has to fill the pairs: by the tile
+        // times, in whole waves (one group of 1024 rows, N 1024, K 7168: 22.0 us on pairs, 18.8).  Layouts sized for the
+        // worst case (a device-side block count, rows stored through addresses) stay on single CTAs.
+        if (plain && forced_cl == 0 && n >= 224u && m >= 6ull * kBlockM * num_groups && m / kBlockM <= kMaxPairedBlocks) {
+            const uint64_t tiles = (uint64_t)ceil_div(m, 2u * kBlockM) * ceil_div(n, 224u);
+            const uint64_t waves = (tiles + sms / 2u - 1u) / (sms / 2u);
+            if ((double)waves * scaled_tile_ns(2u, p.num_k_blocks, times.pair_kb[7]) < single_ns) { cl = 2u; dense_bn = 224u; }
+        }
+    }
     plan->cluster = cl;
     const uint32_t tile_m = kBlockM * cl;
     const uint32_t units = sms / cl;

@@ -429,27 +429,31 @@ def test_config_introspection():
     assert get_gemm_config(Dtype.Bf16, 0, 2048, 2048, 2048)["block_k"] == 64
 
 
-@pytest.mark.parametrize("groups,n,k,blocks", [
-    (2, 224, 512, [0, 0, 0, 1, 1]),                          # one full tile wide, 320 rows per group: the first size on pairs
-    (2, 224, 512, [0, 0, 1, 1]),                             # the last on single CTAs
-    (1, 1000, 1024, [0, 0, 0, -1, 0, 0, -1, 0, 0]),          # narrow last column tile, odd runs, unowned blocks
-    (1, 220, 512, [0] * 9),                                  # narrower than a tile: single CTAs
+@pytest.mark.parametrize("groups,n,k,blocks,cluster", [
+    (2, 224, 512, [0] * 5 + [1] * 7, 2),                     # six blocks per group, one full tile wide: the first size on pairs
+    (2, 224, 512, [0] * 4 + [1] * 7, 1),                     # the last on single CTAs
+    (1, 1000, 512, [0, 0, 0, -1, 0, 0, -1, 0, 0], 2),        # narrow last column tile, odd runs, unowned blocks
+    (1, 1000, 1024, [0, 0, 0, -1, 0, 0, -1, 0, 0], 1),       # too few tiles for pairs at this K
+    (1, 220, 512, [0] * 9, 1),                               # narrower than a tile
 ])
-def test_m_grouped_contiguous_choice_of_pairs(groups, n, k, blocks):
-    """FP8 per-128: layouts of at least 320 rows per group and 224 columns run on CTA pairs with 224-wide tiles.  The result
-    is the same bit for bit as on single CTAs, and unowned blocks stay untouched."""
+def test_m_grouped_contiguous_choice_of_pairs(groups, n, k, blocks, cluster, monkeypatch, capfd):
+    """FP8 per-128: layouts of at least six blocks per group run on CTA pairs with 224-wide tiles where their tiles fill them.
+    The result is the same bit for bit on pairs and on single CTAs, and unowned blocks stay untouched."""
     m = 128 * len(blocks)
     a, ga = quantised_operand(randn((m, k), 21), "fp8", 128)
     b, gb = _stacked_b("fp8", groups, n, k, 22, gran=128)
+    indices = dev(np.array(blocks, dtype=np.int32))
+    monkeypatch.setenv("DG_PRINT_CONFIGS", "1")
     got = []
-    for cluster in (None, "1"):
-        if cluster:
-            os.environ["DG_CLUSTER"] = cluster
+    for forced in (None, "1", "2"):
+        if forced:
+            monkeypatch.setenv("DG_CLUSTER", forced)
         out = new_output(m, n, fill=3.0)
-        m_grouped_gemm_nt_contiguous(a, b, out, dev(np.array(blocks, dtype=np.int32)), groups)
+        m_grouped_gemm_nt_contiguous(a, b, out, indices, groups)
         poll_device_status()
         got.append(to_f32(out))
-    assert np.array_equal(got[0], got[1])
+        assert f"cluster={forced or cluster} " in capfd.readouterr().err
+    assert all(np.array_equal(got[0], g) for g in got[1:])
     for i, e in enumerate(blocks):
         rows = np.arange(128 * i, 128 * (i + 1))
         if e < 0:
