@@ -1321,11 +1321,6 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
     return DG_OK;
 }
 
-static bool pdl_enabled() {
-    static const bool on = env_u32("DG_PDL", 1) != 0;
-    return on;
-}
-
 template <int KIND, int GTYPE, int CL, bool SPLIT = false, bool DYN = false, bool MNM = false, bool SFW = false, bool GA = false>
 static int32_t launch(const Plan& plan, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tsa,
                       const CUtensorMap& tsb, cudaStream_t s) {
@@ -1589,19 +1584,9 @@ static int32_t run_gemm(const dg_operand_t* a, const dg_operand_t* b, dg_output_
         else lst = launch<kBf16, kNormal, 1, true>(plan, ta, tb, tsa, tsb, s);
         if (lst == DG_OK) {
             const size_t threads = (size_t)m * ((n + 3) / 4);
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((uint32_t)((threads + 255) / 256));
-            cfg.blockDim = dim3(256);
-            cfg.stream = s;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = pdl_enabled() ? 1 : 0;
-            cudaError_t e = cudaLaunchKernelEx(&cfg, split_reduce_kernel, (const float*)p.split_ws, p.k_splits, m, n, out->data,
-                                               (uint64_t)out->stride, p.out_f32, p.accumulate, alpha);
+            cudaError_t e = launch_dependent(split_reduce_kernel, (uint32_t)((threads + 255) / 256), 256u, 0u, s, (const float*)p.split_ws, p.k_splits,
+                                             m, n, out->data, (uint64_t)out->stride, p.out_f32, p.accumulate, alpha);
             if (e != cudaSuccess) lst = fail(DG_ERR_DRIVER, "split-K reduction launch failed: %s", cudaGetErrorString(e));
-            else note_launch();
         }
         if (graph_ws) cudaFreeAsync(graph_ws, s);
         return lst;

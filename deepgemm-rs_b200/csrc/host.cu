@@ -3,6 +3,7 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <atomic>
 #include <mutex>
 
@@ -20,6 +21,14 @@ int32_t fail(int32_t code, const char* fmt, ...) {
 
 static std::atomic<unsigned long long> g_launches{0};
 void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+
+bool pdl_enabled() {
+    static const bool on = [] {
+        const char* v = getenv("DG_PDL");
+        return !(v && *v) || strtoul(v, nullptr, 10) != 0;
+    }();
+    return on;
+}
 
 static std::mutex g_mu;
 static DeviceInfo g_dev[64];

@@ -49,6 +49,28 @@ int32_t make_tmap_2d(CUtensorMap* map, CUtensorMapDataType dt, uint32_t elem_byt
 // Counts kernel launches made by this library (dg_launch_count reports it).
 void note_launch();
 
+// Whether launches carry the programmatic-stream-serialization attribute (DG_PDL=0 in the environment: no; read once).
+bool pdl_enabled();
+
+// Programmatic dependent launch of a kernel that waits for its predecessor itself (griddep_wait) and lets its successor
+// set up early; a plain launch when switched off.
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*fn)(Params...), uint32_t grid, uint32_t block, uint32_t smem, cudaStream_t s, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);
+    if (e == cudaSuccess) note_launch();
+    return e;
+}
+
 inline uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 inline uint32_t align_up(uint32_t a, uint32_t b) { return ceil_div(a, b) * b; }
 

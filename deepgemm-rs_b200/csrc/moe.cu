@@ -316,23 +316,6 @@ plan_cluster_kernel(const int32_t* __restrict__ expert_of_row, uint32_t n_rows, 
         }
 }
 
-template <typename... Params, typename... Args>
-static cudaError_t launch_pdl(void (*fn)(Params...), uint32_t grid, uint32_t block, uint32_t smem, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, args...);
-    if (e == cudaSuccess) note_launch();
-    return e;
-}
-
 }  // namespace dg
 
 extern "C" {
@@ -352,7 +335,7 @@ int32_t dg_moe_plan(const int32_t* expert_of_row, uint32_t n_rows, uint32_t num_
     if (st != DG_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (n_rows <= dg::kPlanMaxRows && num_experts <= dg::kPlanMaxExperts) {
-        DG_CUDA_CHECK(dg::launch_pdl(dg::plan_cluster_kernel, dg::kPlanBlocks, dg::kPlanThreads,
+        DG_CUDA_CHECK(dg::launch_dependent(dg::plan_cluster_kernel, dg::kPlanBlocks, dg::kPlanThreads,
                                      (uint32_t)sizeof(int32_t) * (4u * num_experts + 1u), s, expert_of_row, n_rows, num_experts, align,
                                      div, capacity, counts, offsets, slot_src, slot_of_row, block_expert));
         return DG_OK;
@@ -419,7 +402,7 @@ int32_t dg_moe_gather(const void* x, uint64_t x_pitch_bytes, uint32_t row_bytes,
     const dg::DeviceInfo* dev;
     int32_t st = dg::current_device(&dev);
     if (st != DG_OK) return st;
-    DG_CUDA_CHECK(dg::launch_pdl(dg::gather_tokens_kernel, dg::ceil_div(capacity, 32u), 256u, 0u, static_cast<cudaStream_t>(stream),
+    DG_CUDA_CHECK(dg::launch_dependent(dg::gather_tokens_kernel, dg::ceil_div(capacity, 32u), 256u, 0u, static_cast<cudaStream_t>(stream),
                                  static_cast<const uint4*>(x), x_pitch_bytes / 16u, x_sf, sf_cols, sf_rows, slot_src, block_expert, align,
                                  capacity, row_bytes / 16u, static_cast<uint4*>(rows_out), sf_out));
     return DG_OK;

@@ -1107,23 +1107,13 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
         uint32_t* req_first = qb_tokens + num_tokens;
         p.cum = cum; p.qb_tokens = qb_tokens; p.req_first = req_first;
         const uint64_t max_ctx64 = (uint64_t)pg.block_table_stride * pg.page_kv;
-        cudaLaunchConfig_t mcfg = {};
-        mcfg.gridDim = dim3(1);
-        mcfg.blockDim = dim3(kMetaThreads);
-        mcfg.stream = s;
-        cudaLaunchAttribute mattr[1];
-        mattr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        mattr[0].val.programmaticStreamSerializationAllowed = 1;
-        mcfg.attrs = mattr;
-        mcfg.numAttrs = 1;
-        const cudaError_t me = cudaLaunchKernelEx(&mcfg, mqa_paged_metadata_kernel, pg.context_lens, pg.indices, num_tokens, block_q,
-                                                  (uint32_t)(max_ctx64 > 0xffffff00ull ? 0xffffff00ull : max_ctx64), cum, qb_tokens,
-                                                  req_first);
+        const cudaError_t me = launch_dependent(mqa_paged_metadata_kernel, 1u, kMetaThreads, 0u, s, pg.context_lens, pg.indices, num_tokens,
+                                                block_q, (uint32_t)(max_ctx64 > 0xffffff00ull ? 0xffffff00ull : max_ctx64), cum, qb_tokens,
+                                                req_first);
         if (me != cudaSuccess) {
             if (meta_owned) cudaFreeAsync(meta, s);
             return fail(DG_ERR_DRIVER, "mqa_logits metadata launch failed: %s", cudaGetErrorString(me));
         }
-        note_launch();
     }
 
     CUtensorMap tq, tkv, tqsf, tkvsf;
@@ -1150,7 +1140,7 @@ static int32_t run_mqa(const void* q, const void* kv, const uint32_t* q_sf, uint
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // set-up overlaps the previous kernel's tail
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
     cudaError_t e;
     // The variants that move registers from the role warps to the epilogue warpgroups block inside the kernel if the
     // registers the block got at launch do not cover what its warpgroups ask for: refuse the launch instead.

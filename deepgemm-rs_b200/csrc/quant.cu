@@ -259,18 +259,9 @@ static int32_t launch_quant_rows(const void* x, uint32_t m, uint32_t k, void* da
     const uint32_t num_spans = ceil_div(k / G, 4);
     const uint32_t num_row_blocks = ceil_div(sf_cols, R);
     const uint64_t warps = (uint64_t)num_spans * num_row_blocks;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((uint32_t)((warps + 7) / 8));
-    cfg.blockDim = dim3(256);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    DG_CUDA_CHECK(cudaLaunchKernelEx(&cfg, quant_mx_kernel<R, G, FP4, SWIGLU, STOCH, PITCHED>, static_cast<const float*>(x), m, k,
-                                     static_cast<uint8_t*>(data_out), sf_out, sf_cols, num_spans, num_row_blocks, src_pitch, seed, block_expert));
-    note_launch();
+    DG_CUDA_CHECK(launch_dependent(quant_mx_kernel<R, G, FP4, SWIGLU, STOCH, PITCHED>, (uint32_t)((warps + 7) / 8), 256u, 0u, s,
+                                   static_cast<const float*>(x), m, k, static_cast<uint8_t*>(data_out), sf_out, sf_cols, num_spans,
+                                   num_row_blocks, src_pitch, seed, block_expert));
     return DG_OK;
 }
 
