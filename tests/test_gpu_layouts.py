@@ -245,3 +245,22 @@ def test_bf16_mn_major_choice_of_pairs(layout, m, n, k, cluster, monkeypatch, ca
     assert f"cluster={cluster} " in capfd.readouterr().err
     ref = x.double() @ w.double().t()
     assert (out.data.double() - ref).abs().max().item() <= k * 2.0 ** -24 * k ** 0.5 + 1e-4
+
+
+@pytest.mark.parametrize("cluster", [None, "2"])
+@pytest.mark.parametrize("kind,batch,m,n,k,gran", [("fp4", 3, 300, 520, 512, 32), ("fp4", 2, 129, 200, 1024, 32), ("fp8", 2, 257, 1000, 640, 32),
+                                                   ("fp8", 3, 512, 264, 512, 32)])
+def test_bmm_with_several_row_blocks(kind, batch, m, n, k, gran, cluster, monkeypatch):
+    """Batches of more than 128 rows with scale factors on every k-block, on the chosen tiles and on CTA pairs: ragged rows and
+    columns next to another batch's."""
+    if cluster:
+        monkeypatch.setenv("DG_CLUSTER", cluster)
+    test_bmm_over_batched_sf_arenas(kind, batch, m, n, k, gran)
+
+
+@pytest.mark.parametrize("fp4_side", ["a", "b"])
+@pytest.mark.parametrize("m,n,k,gran8", [(129, 200, 512, 32), (300, 1000, 768, 128), (640, 2048, 1024, 128)])
+def test_mixed_fp8_fp4_operands_on_cta_pairs(fp4_side, m, n, k, gran8, monkeypatch):
+    """The unpacking copies of a pair: half of B per CTA, whose bytes the leader's barrier counts as read, not as written."""
+    monkeypatch.setenv("DG_CLUSTER", "2")
+    test_mixed_fp8_fp4_operands(fp4_side, m, n, k, gran8)
