@@ -597,8 +597,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         }
     } else if (warp == 2 && kHasSf) {
         // ===================================================== SF warp: transposes the SF rows in shared memory and copies them into tensor memory
-        // With SFW the copies (tcgen05.cp) are issued here, not by the MMA issuer: each costs the issuing thread
-        // some 200 cycles, and the MMA issuer's loop, not the tensor pipe, bounded the single-CTA kernel.  Two sets of SF columns
+        // With SFW the copies (tcgen05.cp) are issued here, not by the MMA issuer, whose loop, not the tensor pipe, bounded
+        // the single-CTA kernel while the copies were loops of some 200 cycles each.  Straight-line they cost less, and copied
+        // by the issuer 4096 x 7168 x 7168 on 208 columns takes 175.6 us against 173.3 here.  Two sets of SF columns
         // take turns; the set written for SF k-block n was last read by the MMAs of SF k-block n - 2, whose
         // completion the MMA issuer reports on sf_free.  (Single CTAs only: on a pair the copy reads both CTAs'
         // shared memory, the leader's warp would have to wait for its partner, and that measured slower.)
@@ -1136,7 +1137,7 @@ static uint32_t pick_block_n(int kind, uint32_t m_tiles_total, uint32_t n, uint3
 struct TileTimes { double single_kb[8], pair_kb[8]; };    // 0: not measured, not offered
 static const uint32_t kTileWidths[8] = {64, 96, 128, 160, 176, 192, 208, 224};
 static const TileTimes kFp8Per128 = {{181, 200, 248, 302, 331, 328, 369, 429}, {194, 210, 233, 277, 0, 302, 336, 367}};
-static const TileTimes kFp8Per32 = {{231, 228, 254, 322, 0, 344, 376, 441}, {0, 268, 279, 322, 0, 332, 363, 384}};    // either operand per 32
+static const TileTimes kFp8Per32 = {{231, 228, 254, 322, 0, 344, 376, 441}, {0, 268, 279, 322, 0, 332, 363, 384}};    // either operand per 32; FP8 x FP4 too (60 shapes: none slower than by the formula before)
 static const TileTimes kFp4Times = {{214, 231, 254, 324, 0, 320, 354, 392}, {0, 303, 305, 363, 0, 364, 378, 385}};
 static double scaled_tile_ns(uint32_t cl, uint32_t kb, double per_kb) { return (cl == 1 ? 1300.0 : 400.0) + kb * per_kb; }
 static double pick_scaled_tile(const TileTimes& times, uint32_t m, uint32_t groups, uint32_t n, uint32_t kb, uint32_t sms, uint32_t* cl_out,
@@ -1234,7 +1235,8 @@ static int32_t make_plan(int kind, int gtype, uint32_t m, uint32_t n, uint32_t k
         // Cost of a (tile width, K ranges) choice in nanoseconds, fitted to a sweep on B200 (M = 128, rotating
         // weights): the longer of the busiest CTA's k-loop (its k-blocks x the measured time per k-block of that
         // width) and the weight stream from DRAM, a fixed part per wave, and the second kernel: a fixed part plus
-        // one pass over the f32 partial tiles per range.  Few ranges on narrow tiles beat many on wide ones.
+        // one pass over the f32 partial tiles per range.  Few ranges on narrow tiles beat many on wide ones.  (The
+        // times per k-block are of that sweep; those of kFp8Per128 are later ones, under the power cap.)
         const uint32_t forced_bn = env_u32("DG_BLOCK_N", 0);
         uint32_t best_bn = p.block_n, best_splits = 1;
         double best_cost = 1e30;

@@ -48,8 +48,9 @@ __global__ void __launch_bounds__(256) gather_sf_kernel(const uint32_t* __restri
 // of its packed scale factors (zeros for idx[i] < 0).  A block owns 32 slots: every warp copies four rows, one vector of
 // each in flight at a time and two vectors deep, then the words of every eighth scale-factor row, one slot per lane.
 // Slots of blocks that no expert owns (block_expert < 0) are left as they are: the GEMM visits none of them.
-// HBM-bound by the rows written (the rows read are a top-k-th of them and stay in L2): 163584 slots of 7168 bytes, a
-// tenth of them unowned, 291 us where gather_rows and gather_sf took 290.
+// HBM-bound by the rows written (the rows read are a top-k-th of them and stay in L2).  Against gather_rows and gather_sf,
+// which write the unowned blocks too: 163584 slots of 7168 bytes, a tenth of them unowned, 278 us and 294; 24320 of 7168 29
+// and 38; 49024 of 4096 32 and 40; 2304 of 2048 11 and 18 (launches).
 __global__ void __launch_bounds__(256) gather_tokens_kernel(const uint4* __restrict__ x, uint64_t x_pitch_vec, const uint32_t* __restrict__ sf,
                                                            uint64_t sf_cols, uint32_t sf_rows, const int32_t* __restrict__ idx,
                                                            const int32_t* __restrict__ block_expert, uint32_t block_rows, uint32_t n,
@@ -199,7 +200,8 @@ __global__ void __launch_bounds__(256) plan_place_kernel(const int32_t* __restri
 // its block's rows, so placing needs no second atomic.  The blocks read one another's counts through distributed
 // shared memory, each scans all experts for itself, and slot = offset of the expert + rows of the blocks before + rank.
 // The padding slots are filled here too.  Bound by launch and latency, not by bytes; two fills and the three kernels
-// below took 61 us for 131072 rows and 256 experts and 19 us for 16152 rows and 64 experts, this one 21 and 12 us.
+// below took 61 us for 131072 rows and 256 experts and 19 us for 16152 rows and 64 experts, this one 21 and 12 us.  Rows are
+// held in registers, which ends it at 131072; beyond, the fills and kernels below cost some 40 us more.
 constexpr uint32_t kPlanBlocks = 8, kPlanThreads = 1024, kPlanRows = 16;
 constexpr uint32_t kPlanMaxRows = kPlanBlocks * kPlanThreads * kPlanRows;
 constexpr uint32_t kPlanMaxExperts = 2048;

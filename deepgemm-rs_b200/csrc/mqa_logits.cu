@@ -184,16 +184,6 @@ struct MqaTasks {
     }
 };
 
-// Row of the paged cache that holds token `tok` (request order) of the request whose table row is given;
-// tokens past the table's width or pages outside the cache read row 0 (they lie beyond every context
-// length and are masked by the epilogue).
-__device__ __forceinline__ uint32_t paged_row(const MqaParams& p, uint32_t table_row, uint32_t tok, uint32_t span) {
-    const uint32_t pg = tok / p.page_kv;
-    const uint32_t page = pg < p.block_table_stride ? __ldg(p.block_table + (size_t)table_row * p.block_table_stride + pg) : 0u;
-    const uint32_t row = page * p.page_kv + tok % p.page_kv;
-    return row + span <= p.num_kv ? row : 0u;
-}
-
 __device__ __forceinline__ void tc_mma_f8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -336,7 +326,8 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         if (!(ok = DG_WARP_WAIT(smem_u32(&bars->kv_empty[stage]), phase ^ 1u, wc, kWaitEmpty))) break;
                         const uint32_t bar = smem_u32(&bars->kv_full[stage]);
                         const uint32_t dst = base + p.off_kv + stage * p.kv_stage_bytes;
-                        // rows past the table's width or pages outside the cache read row 0 (paged_row)
+                        // tokens past the table's width or pages outside the cache read row 0: they lie beyond every
+                        // context length and are masked by the epilogue
                         uint32_t row = pq[j] * p.page_kv + (tok_of(kb) & (p.page_kv - 1u));
                         if (row + p.box_rows > p.num_kv) row = 0u;
                         pq[j] = page_of(kb + kPagesAhead);
@@ -472,9 +463,9 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     } else if (warp == 2 && SCALED) {
         // ===================================================== scale factors (ue8m0 contracts)
         // tcgen05.cp wants the word of row 32 i + l at position 4 l + i.  Contiguous kv: the TMA load
-        // brought the 128 words in row order, rewrite them in place.  Paged kv: the words are fetched
-        // here, page by page with plain loads (a page's words may be fewer than a TMA box can address),
-        // as soon as the stage is free, and stored in the final order directly.
+        // brought the 128 words in row order, rewrite them in place.  Paged kv: the words are copied
+        // here (cp.async; a page's words may be fewer than a TMA box can address) as soon as the stage
+        // is free, straight to their final order.
         uint32_t stage = 0, phase = 0, qcount = 0;
         bool ok = true;
         auto transpose128 = [&](uint32_t* q) {
