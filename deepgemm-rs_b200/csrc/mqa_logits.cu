@@ -454,9 +454,11 @@ mqa_logits_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 stage = __shfl_sync(0xffffffffu, stage, issuer_lane);
                 phase = __shfl_sync(0xffffffffu, phase, issuer_lane);
                 acount = __shfl_sync(0xffffffffu, acount, issuer_lane);
-                acc_bits = __shfl_sync(0xffffffffu, acc_bits, issuer_lane);
-                ring = __shfl_sync(0xffffffffu, ring, issuer_lane);
-                ring_q = __shfl_sync(0xffffffffu, ring_q, issuer_lane);
+                if (DEC) {      // (elsewhere they would live in registers that the role warps do not have)
+                    acc_bits = __shfl_sync(0xffffffffu, acc_bits, issuer_lane);
+                    ring = __shfl_sync(0xffffffffu, ring, issuer_lane);
+                    ring_q = __shfl_sync(0xffffffffu, ring_q, issuer_lane);
+                }
                 ok = __shfl_sync(0xffffffffu, (uint32_t)ok, issuer_lane) != 0u;
             }
         }
