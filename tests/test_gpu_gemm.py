@@ -464,9 +464,11 @@ def test_m_grouped_contiguous_choice_of_pairs(groups, n, k, blocks, cluster, mon
 
 @pytest.mark.parametrize("kind,gran", [("fp8", 32), ("fp4", 32)])
 @pytest.mark.parametrize("m,n,k", [(129, 200, 768), (300, 1000, 2304), (512, 2560, 512)])
-def test_scale_factors_on_every_k_block_on_pairs(kind, gran, m, n, k):
-    """FP8 per-32 and FP4 with more than one row block run on CTA pairs: ragged rows, a second CTA with one row, narrow tiles."""
-    run_dense(kind, m, n, k, gran_a=gran, gran_b=gran, seed=m + n)
+@pytest.mark.parametrize("cluster", [None, 2])
+def test_scale_factors_on_every_k_block_on_pairs(kind, gran, m, n, k, cluster):
+    """FP8 per-32 and FP4 with more than one row block, on the tiles the library chooses and on CTA pairs: ragged rows, a second
+    CTA with one row, narrow tiles."""
+    run_dense(kind, m, n, k, gran_a=gran, gran_b=gran, seed=m + n, cluster=cluster)
 
 
 @pytest.mark.parametrize("kind,gran", [("fp8", 128), ("fp8", 32), ("fp4", 32)])
